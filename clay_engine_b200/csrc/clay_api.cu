@@ -236,9 +236,45 @@ struct clay_splat {
   uint32_t* keys = nullptr;
   SplatDev h{};
   SplatDev* d = nullptr;          // cloud in index order
-  SplatDev* d_ordered = nullptr;  // the fluid's cloud in cell order (fluid-owned splats)
+  // fluid-owned splats: the fluid's cloud in cell order, as the splat (d_plain) and the gather see it
+  SplatDev *d_plain = nullptr, *d_ordered = nullptr;
   const uint32_t* order = nullptr;
+  // A fluid's surface may be baked by gathering over a box tree of the cell-ordered cloud, in
+  // scratch that the fluid's neighbour lists leave free once the last substep has read them.
+  float4* tree = nullptr;
+  bool sorted = false;  // gathered in Morton order
+  const GridState* gs = nullptr;
   bool desc_dirty = true;
+
+  // Blocks of 8 x 4 x 2 voxels over all levels: the most a bake's list holds.
+  int64_t blocks() const { return vol->total / 64; }
+  // `gather`: the device chooses how to bake it, else it is splatted.
+  void bind_tree(SplatDev* o, bool gather) const {
+    o->order = order;
+    if (!gather || cloud.capacity < kGatherMin) return;
+    const BakeTreeLayout l = bake_tree_layout(cloud.capacity);
+    o->gs = gs;
+    o->bpos = tree;
+    o->leaf = tree + l.leaf;
+    o->group = tree + l.group;
+    o->super = tree + l.super;
+    o->cursor = sorted ? reinterpret_cast<uint32_t*>(tree + l.cursor) : nullptr;
+  }
+  // Whether `live` particles baked by themselves are gathered (bake_gathers' second rule, which they then fulfil).
+  bool gathers(int64_t live) const {
+    return gs && live >= kGatherAlone && 8 * live >= static_cast<int64_t>(res) * res * res && list(blocks()).items;
+  }
+  // A bake list of `items` blocks in what the tree leaves of the neighbour lists' memory (NULL where it does not fit).
+  BakeList list(int64_t items) const {
+    const uint64_t at = bake_tree_layout(cloud.capacity).list, slots = static_cast<uint64_t>(cloud.capacity) * (kMaxNbr / 4);
+    if (items > (int64_t{1} << 31) || at * 16 + kListCounterBytes + 8 * static_cast<uint64_t>(items) > slots * 16) return {nullptr, nullptr, 0u};
+    char* p = reinterpret_cast<char*>(tree + at);
+    return {reinterpret_cast<uint2*>(p + kListCounterBytes), reinterpret_cast<uint32_t*>(p), static_cast<uint32_t>(items)};
+  }
+  // Parts of the bake order's scan: as many bins as the cloud can have.
+  int sort_parts() const {
+    return static_cast<int>((std::min<int64_t>(kSortBins, cloud.capacity) + 1 + kSortPart - 1) / kSortPart);
+  }
 
   int flush(cudaStream_t s) {
     int rc = vol->flush(s);
@@ -249,7 +285,10 @@ struct clay_splat {
     if (rc) return rc;
     if (d_ordered) {
       SplatDev o = h;
-      o.order = order;
+      bind_tree(&o, false);
+      rc = ctx->upload(d_plain, &o, sizeof(o), s);
+      if (rc) return rc;
+      bind_tree(&o, true);
       rc = ctx->upload(d_ordered, &o, sizeof(o), s);
       if (rc) return rc;
     }
@@ -475,8 +514,9 @@ int make_splat(clay_ctx* ctx, const clay_cloud_desc* cloud, const clay_splat_opt
   if ((rc = ctx->dev_alloc(&p, sizeof(SplatDev)))) goto fail_out;
   s->d = static_cast<SplatDev*>(p);
   if (with_order) {
-    if ((rc = ctx->dev_alloc(&p, sizeof(SplatDev)))) goto fail_out;
-    s->d_ordered = static_cast<SplatDev*>(p);
+    if ((rc = ctx->dev_alloc(&p, 2 * sizeof(SplatDev)))) goto fail_out;
+    s->d_plain = static_cast<SplatDev*>(p);
+    s->d_ordered = s->d_plain + 1;
   }
   {
     SplatDev& h = s->h;
@@ -521,7 +561,7 @@ int make_splat(clay_ctx* ctx, const clay_cloud_desc* cloud, const clay_splat_opt
 fail_out:
   if (s->keys) ctx->dev_free(s->keys, sizeof(uint32_t) * vol->total);
   if (s->d) ctx->dev_free(s->d, sizeof(SplatDev));
-  if (s->d_ordered) ctx->dev_free(s->d_ordered, sizeof(SplatDev));
+  if (s->d_plain) ctx->dev_free(s->d_plain, 2 * sizeof(SplatDev));
   free_field(s->field);
   free_volume(vol);
   delete s;
@@ -532,18 +572,34 @@ void free_splat(clay_splat* s) {
   if (!s) return;
   s->ctx->dev_free(s->keys, sizeof(uint32_t) * s->vol->total);
   s->ctx->dev_free(s->d, sizeof(SplatDev));
-  if (s->d_ordered) s->ctx->dev_free(s->d_ordered, sizeof(SplatDev));
+  if (s->d_plain) s->ctx->dev_free(s->d_plain, 2 * sizeof(SplatDev));
   free_field(s->field);
   free_volume(s->vol);
   delete s;
 }
 
-// Blocks over the cloud's iteration space for every mip (plain bake).
-int splat_bake(clay_splat* s, cudaStream_t st, bool ordered, int64_t iter_n) {
+// Chunks of 8^3 voxels over all levels, in blocks of the mark pass.
+int mark_blocks(const clay_splat* s) { return static_cast<int>((s->vol->total / 512 + kMarkChunks - 1) / kMarkChunks); }
+
+// Blocks over the cloud's iteration space for every mip (plain bake), of a fluid (`scene`) in cell
+// order; a large fluid is gathered.
+int splat_bake(clay_splat* s, cudaStream_t st, const SceneDev* scene, int64_t iter_n) {
   int rc = s->flush(st);
   if (rc) return rc;
-  const SplatDev* d = (ordered && s->d_ordered) ? s->d_ordered : s->d;
   int64_t n = iter_n;
+  if (scene && s->gathers(n)) {
+    const BakeList list = s->list(s->blocks());
+    if (s->sorted) {
+      CK(L_sort_scan(scene, s->d_ordered, nullptr, s->sort_parts(), false, st));
+      CK(L_sort_scan(scene, s->d_ordered, nullptr, s->sort_parts(), true, st));
+      CK(L_sort_scatter(scene, s->d_ordered, nullptr, static_cast<int>((n + 255) / 256), st));
+    }
+    CK(L_bake_tree(s->d_ordered, nullptr, static_cast<int>((n + kGroupN - 1) / kGroupN), list, st));
+    CK(L_bake_mark(s->d_ordered, nullptr, mark_blocks(s), list, st));
+    CK(L_bake_gather(s->d_ordered, static_cast<int>(std::min<int64_t>(kGatherBlocks, s->blocks())), list, st));
+    return CLAY_OK;
+  }
+  const SplatDev* d = scene ? s->d_plain : s->d;
   if (n > 0) {
     int blocks = static_cast<int>((n + kSplatThreads - 1) / kSplatThreads);
     CK(L_splat(d, nullptr, blocks, s->mips, s->cloud.normals ? kSplatAccVoxelsDiscs : kSplatAccVoxels, st));
@@ -849,7 +905,7 @@ int clay_splat_set_center(clay_splat* s, double x, double y, double z) {
 
 int clay_splat_bake(clay_splat* s, void* stream) {
   if (!s) return fail(CLAY_EINVAL, "clay_splat_bake: NULL splat");
-  return splat_bake(s, static_cast<cudaStream_t>(stream), false, s->cloud.capacity);
+  return splat_bake(s, static_cast<cudaStream_t>(stream), nullptr, s->cloud.capacity);
 }
 
 clay_volume* clay_splat_volume(clay_splat* s) { return s ? s->vol : nullptr; }
@@ -967,7 +1023,7 @@ int clay_fluid_estimate_bytes(const clay_fluid_opts* opts, uint64_t* out) {
     t += r * r * r;
   }
   // volume planes (f16 distance, f16 material) and uniform, its field, the key grid, descriptors
-  b += t * (2 * sizeof(__half) + sizeof(uint32_t)) + sizeof(VolParamsDev) + sizeof(FieldDev) + 2 * sizeof(SplatDev);
+  b += t * (2 * sizeof(__half) + sizeof(uint32_t)) + sizeof(VolParamsDev) + sizeof(FieldDev) + 3 * sizeof(SplatDev);
   *out = b;
   return CLAY_OK;
 }
@@ -1072,6 +1128,9 @@ int clay_fluid_create(clay_ctx* ctx, const clay_field* world, const clay_fluid_o
     return rc;
   }
   f->surface->order = f->hs.sorted_id;
+  f->surface->tree = reinterpret_cast<float4*>(f->hs.nbr);
+  f->surface->sorted = f->substeps > 0 && C > kSortMin;
+  f->surface->gs = f->substeps > 0 ? f->gs : nullptr;  // without substeps there is no cell order
   f->surface->desc_dirty = true;
   rc = f->surface->flush(nullptr);
   if (rc) {
@@ -1196,7 +1255,7 @@ int clay_fluid_step(clay_fluid* f, void* stream) {
     if (rc) return rc;
   }
   bool ordered = f->substeps > 0 && f->live > 0;
-  return splat_bake(f->surface, s, ordered, ordered ? f->live : f->capacity);
+  return splat_bake(f->surface, s, ordered ? f->d_scene : nullptr, ordered ? f->live : f->capacity);
 }
 
 int64_t clay_fluid_particle_count(const clay_fluid* f) { return f ? f->live : -1; }
@@ -1361,9 +1420,12 @@ struct clay_batch {
   size_t n_scenes_alloc = 0;
   SplatDev* d_extra = nullptr;   // extra clouds, index order
   SplatDev* d_surf = nullptr;    // fluid surfaces, cell order
-  Work *w_part = nullptr, *w_emit = nullptr, *w_scan = nullptr, *w_xsplat = nullptr, *w_xres = nullptr,
-       *w_ssplat = nullptr, *w_sres = nullptr;
-  int n_part = 0, n_emit = 0, n_scan = 0, n_xsplat = 0, n_xres = 0, n_ssplat = 0, n_sres = 0;
+  SplatDev* d_surf_splat = nullptr;  // the same, always splatted
+  Work *w_emit = nullptr, *w_scan = nullptr, *w_xsplat = nullptr, *w_xres = nullptr,
+       *w_ssplat = nullptr, *w_sres = nullptr, *w_sort = nullptr, *w_scatter = nullptr, *w_tree = nullptr, *w_mark = nullptr;
+  int n_part = 0, n_emit = 0, n_scan = 0, n_xsplat = 0, n_xres = 0, n_ssplat = 0, n_sres = 0, n_sort = 0, n_scatter = 0, n_tree = 0, n_mark = 0;
+  int n_gather = 0;
+  bool gather = false;  // the device chooses per scene between the splat and the gather
   std::vector<DevBuf> bufs;
   bool built = false;
   cudaGraphExec_t graph = nullptr;
@@ -1388,8 +1450,9 @@ struct clay_batch {
   // so one lane's latency-bound passes overlap another's issue-bound ones and each pass's tail.
   struct Lane {
     std::vector<PartGroup> groups;
-    Work *w_emit = nullptr, *w_scan = nullptr, *w_ssplat = nullptr, *w_sres = nullptr;
-    int n_part = 0, n_emit = 0, n_scan = 0, n_ssplat = 0, n_sres = 0;
+    Work *w_emit = nullptr, *w_scan = nullptr, *w_ssplat = nullptr, *w_sres = nullptr, *w_sort = nullptr, *w_scatter = nullptr, *w_tree = nullptr, *w_mark = nullptr;
+    int n_part = 0, n_emit = 0, n_scan = 0, n_ssplat = 0, n_sres = 0, n_sort = 0, n_scatter = 0, n_tree = 0, n_mark = 0, n_gather = 0;
+    BakeList list{};
     cudaStream_t stream = nullptr;  // lane 0 runs on the frame's stream
     cudaEvent_t done = nullptr;
   };
@@ -1471,14 +1534,37 @@ struct clay_batch {
     bufs.clear();
     built = false;
   }
+  // The tables share one allocation, filled on the host and uploaded in one copy (40 allocations and copies
+  // were most of a batch's first frame): reserved for `bytes` of them, then each placed by upload_table.
+  char* arena = nullptr;
+  std::vector<char> stage;
+  size_t staged = 0;
+  template <class T>
+  static size_t table_bytes(size_t n) {
+    return (sizeof(T) * std::max<size_t>(n, 1) + 255) / 256 * 256;
+  }
+  int reserve_tables(size_t bytes) {
+    void* p = nullptr;
+    int rc = ctx->dev_alloc(&p, bytes);
+    if (rc) return rc;
+    bufs.push_back({p, bytes});
+    arena = static_cast<char*>(p);
+    stage.assign(bytes, 0);
+    staged = 0;
+    return CLAY_OK;
+  }
   template <class T>
   int upload_table(T** d, const std::vector<T>& h) {
-    void* p = nullptr;
-    int rc = ctx->dev_alloc(&p, sizeof(T) * std::max<size_t>(h.size(), 1));
-    if (rc) return rc;
-    bufs.push_back({p, sizeof(T) * std::max<size_t>(h.size(), 1)});
-    if (!h.empty()) CK(cudaMemcpy(p, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice));
-    *d = static_cast<T*>(p);
+    const size_t n = table_bytes<T>(h.size());
+    if (staged + n > stage.size()) return fail(CLAY_ESTATE, "clay_batch: tables beyond their reservation");
+    if (!h.empty()) std::memcpy(stage.data() + staged, h.data(), sizeof(T) * h.size());
+    *d = reinterpret_cast<T*>(arena + staged);
+    staged += n;
+    return CLAY_OK;
+  }
+  int upload_staged() {
+    CK(cudaMemcpy(arena, stage.data(), staged, cudaMemcpyHostToDevice));
+    stage = std::vector<char>();
     return CLAY_OK;
   }
 };
@@ -1493,6 +1579,34 @@ void add_splat_work(std::vector<Work>& ws, std::vector<Work>& wr, uint32_t obj, 
                     static_cast<uint32_t>(std::min<int64_t>(splat_block, iter_n - f))});
   int64_t quads = (s->vol->total + 3) / 4;
   for (int64_t q = 0; q < quads; q += kResolveThreads) wr.push_back({obj, 0u, static_cast<uint32_t>(q), kResolveThreads});
+}
+
+// The gather bake of surface `obj`: for a large scene the parts of its sort and its particles,
+// then tree groups over `iter_n` particles, marks over all levels.
+void add_bake_work(std::vector<Work>& wo, std::vector<Work>& wc, std::vector<Work>& wt, std::vector<Work>& wm, uint32_t obj, const clay_splat* s, int64_t iter_n) {
+  if (s->sorted && iter_n > 0) {
+    for (int p = 0; p < s->sort_parts(); p++) wo.push_back({obj, static_cast<uint32_t>(p), 0u, 0u});
+    for (int64_t f = 0; f < iter_n; f += 256)
+      wc.push_back({obj, 0u, static_cast<uint32_t>(f), static_cast<uint32_t>(std::min<int64_t>(256, iter_n - f))});
+  }
+  for (int64_t f = 0; f < iter_n; f += kGroupN) wt.push_back({obj, 0u, static_cast<uint32_t>(f), kGroupN});
+  for (int k = 0; k < mark_blocks(s); k++)
+    wm.push_back({obj, 0u, static_cast<uint32_t>(k * kMarkChunks), static_cast<uint32_t>(kMarkChunks)});
+}
+
+// The bake list of the scenes stepped together (indices into the batch), in the memory of the largest of
+// them; items == NULL where it does not fit (small scenes with large volumes), which are then splatted.
+template <class Scenes>
+BakeList batch_list(const clay_batch* b, const Scenes& scenes) {
+  const clay_splat* largest = nullptr;
+  int64_t items = 0;
+  for (int i : scenes) {
+    const clay_splat* s = b->sims[static_cast<size_t>(i)]->surface;
+    if (!s->gs || s->cloud.capacity < kGatherMin) continue;
+    items += s->blocks();
+    if (!largest || s->cloud.capacity > largest->cloud.capacity) largest = s;
+  }
+  return largest ? largest->list(items) : BakeList{nullptr, nullptr, 0u};
 }
 
 // Work tables sized by capacity: blocks past a scene's live count exit at once, so the
@@ -1528,8 +1642,34 @@ int batch_build(clay_batch* b) {
     for (int e = 0; e < eb; e++) we.push_back({obj, 0u, static_cast<uint32_t>(e * T), static_cast<uint32_t>(eb * T)});
     for (uint32_t p = 0; p < f->parts_scan; p++) wsc.push_back({obj, p, 0u, 0u});
   }
-  std::vector<SplatDev> xs, ss;
-  std::vector<Work> wxs, wxr, wss, wsr;
+  std::vector<SplatDev> xs, ss, sp;
+  std::vector<Work> wxs, wxr, wss, wsr, wso, wsc2, wtr, wmk;
+  int64_t items = 0, particles = 0;
+  for (const clay_fluid* f : b->sims) particles += f->capacity;
+  // lanes: scenes dealt largest first to the lane with the fewest particles so far
+  const int nl = std::max(1, std::min(b->n_lanes, static_cast<int>(std::max<size_t>(b->sims.size(), 1))));
+  std::vector<int> lane_of(b->sims.size(), 0);
+  std::vector<std::vector<int>> of_lane(static_cast<size_t>(nl));
+  {
+    std::vector<int64_t> load(static_cast<size_t>(nl), 0);
+    std::vector<size_t> by_size(b->sims.size());
+    for (size_t i = 0; i < by_size.size(); i++) by_size[i] = i;
+    std::stable_sort(by_size.begin(), by_size.end(),
+                     [&](size_t x, size_t y) { return b->sims[x]->capacity > b->sims[y]->capacity; });
+    for (size_t i : by_size) {
+      const int l = static_cast<int>(std::min_element(load.begin(), load.end()) - load.begin());
+      lane_of[i] = l;
+      of_lane[static_cast<size_t>(l)].push_back(static_cast<int>(i));
+      load[static_cast<size_t>(l)] += b->sims[i]->capacity;
+    }
+  }
+  b->gather = particles >= kGatherBatch;
+  for (const std::vector<int>& l : of_lane) b->gather = b->gather && batch_list(b, l).items;
+  {
+    std::vector<int> all(b->sims.size());
+    for (size_t i = 0; i < all.size(); i++) all[i] = static_cast<int>(i);
+    b->gather = b->gather && batch_list(b, all).items;  // clay_batch_profile steps them in one lane
+  }
   for (size_t i = 0; i < b->extra.size(); i++) {
     xs.push_back(b->extra[i]->h);
     xs.back().order = nullptr;
@@ -1538,14 +1678,26 @@ int batch_build(clay_batch* b) {
   for (size_t i = 0; i < b->sims.size(); i++) {
     clay_splat* s = b->sims[i]->surface;
     SplatDev d = s->h;
-    d.order = s->order;
+    s->bind_tree(&d, b->gather);
     const clay_bucket_tuning bt = b->tuning_of(b->sims[i]->capacity);
     d.tile_ratio = static_cast<uint32_t>(bt.splat_tile_ratio);
     d.walk_weight = static_cast<uint32_t>(bt.splat_walk_weight);
     ss.push_back(d);
     add_splat_work(wss, wsr, static_cast<uint32_t>(i), s, b->sims[i]->capacity, kSplatThreads);
+    if (!d.gs) continue;
+    add_bake_work(wso, wsc2, wtr, wmk, static_cast<uint32_t>(i), s, b->sims[i]->capacity);
+    items += s->blocks();
   }
   int rc;
+  {
+    size_t works = 0;  // every Work table, by itself and (with more than one lane) once more over the lanes
+    for (const auto* w : {&wp, &we, &wsc, &wss, &wsr, &wso, &wsc2, &wtr, &wmk, &wxs, &wxr}) works += w->size();
+    const size_t tables = static_cast<size_t>(nl + 1) * (blocks.size() + 12);
+    const size_t bytes = (nl > 1 ? 2 : 1) * works * sizeof(Work) + tables * 256 + clay_batch::table_bytes<ParamsDev>(b->sims.size()) +
+                         clay_batch::table_bytes<ContactsDev>(b->sims.size()) + clay_batch::table_bytes<SceneDev>(scenes.size()) +
+                         clay_batch::table_bytes<SplatDev>(xs.size()) + 2 * clay_batch::table_bytes<SplatDev>(ss.size());
+    if ((rc = b->reserve_tables(bytes))) return rc;
+  }
   {
     std::vector<ParamsDev> prm(b->sims.size());
     for (size_t i = 0; i < b->sims.size(); i++) std::memcpy(&prm[i], &b->sims[i]->frozen, sizeof(ParamsDev));
@@ -1556,16 +1708,20 @@ int batch_build(clay_batch* b) {
       scenes[i].prm = b->d_params + i;
       ss[i].live_count = &b->d_params[i].count;
     }
+    sp = ss;
+    for (SplatDev& d : sp) d.gs = nullptr;
     for (int k = 0; k < 2; k++) {
       CK(cudaMallocHost(&b->h_params[k], sizeof(ParamsDev) * std::max<size_t>(b->sims.size(), 1)));
       if (!b->params_ev[k]) CK(cudaEventCreateWithFlags(&b->params_ev[k], cudaEventDisableTiming));
     }
   }
-  if ((rc = b->upload_table(&b->d_scenes, scenes)) || (rc = b->upload_table(&b->w_part, wp)) ||
+  if ((rc = b->upload_table(&b->d_scenes, scenes)) ||
       (rc = b->upload_table(&b->w_emit, we)) || (rc = b->upload_table(&b->w_scan, wsc)) ||
-      (rc = b->upload_table(&b->d_extra, xs)) || (rc = b->upload_table(&b->d_surf, ss)) ||
+      (rc = b->upload_table(&b->d_extra, xs)) || (rc = b->upload_table(&b->d_surf, ss)) || (rc = b->upload_table(&b->d_surf_splat, sp)) ||
       (rc = b->upload_table(&b->w_xsplat, wxs)) || (rc = b->upload_table(&b->w_xres, wxr)) ||
-      (rc = b->upload_table(&b->w_ssplat, wss)) || (rc = b->upload_table(&b->w_sres, wsr)))
+      (rc = b->upload_table(&b->w_sort, wso)) || (rc = b->upload_table(&b->w_scatter, wsc2)) ||
+      (rc = b->upload_table(&b->w_ssplat, wss)) || (rc = b->upload_table(&b->w_sres, wsr)) ||
+      (rc = b->upload_table(&b->w_tree, wtr)) || (rc = b->upload_table(&b->w_mark, wmk)))
     return rc;
   b->n_part = static_cast<int>(wp.size());
   b->groups.clear();
@@ -1575,20 +1731,7 @@ int batch_build(clay_batch* b) {
     b->groups.push_back({w, static_cast<int>(by_block[g].size()), std::get<0>(blocks[g]), std::get<1>(blocks[g]),
                          std::get<2>(blocks[g]) != 0});
   }
-  // lanes: scenes dealt largest first to the lane with the fewest particles so far
   {
-    const int nl = std::max(1, std::min(b->n_lanes, static_cast<int>(std::max<size_t>(b->sims.size(), 1))));
-    std::vector<int> lane_of(b->sims.size(), 0);
-    std::vector<int64_t> load(static_cast<size_t>(nl), 0);
-    std::vector<size_t> by_size(b->sims.size());
-    for (size_t i = 0; i < by_size.size(); i++) by_size[i] = i;
-    std::stable_sort(by_size.begin(), by_size.end(),
-                     [&](size_t x, size_t y) { return b->sims[x]->capacity > b->sims[y]->capacity; });
-    for (size_t i : by_size) {
-      const int l = static_cast<int>(std::min_element(load.begin(), load.end()) - load.begin());
-      lane_of[i] = l;
-      load[static_cast<size_t>(l)] += b->sims[i]->capacity;
-    }
     const size_t old_lanes = b->lanes.size();
     for (size_t l = static_cast<size_t>(nl); l < old_lanes; l++) {
       if (b->lanes[l].stream) cudaStreamDestroy(b->lanes[l].stream);
@@ -1606,6 +1749,20 @@ int batch_build(clay_batch* b) {
       };
       ln.groups.clear();
       ln.n_part = 0;
+      if (nl == 1) {  // one lane: every scene, in the batch's own tables
+        ln.groups = b->groups;
+        ln.n_part = b->n_part;
+        ln.w_emit = b->w_emit, ln.n_emit = static_cast<int>(we.size());
+        ln.w_scan = b->w_scan, ln.n_scan = static_cast<int>(wsc.size());
+        ln.w_ssplat = b->w_ssplat, ln.n_ssplat = static_cast<int>(wss.size());
+        ln.w_sres = b->w_sres, ln.n_sres = static_cast<int>(wsr.size());
+        ln.w_sort = b->w_sort, ln.n_sort = static_cast<int>(wso.size());
+        ln.w_scatter = b->w_scatter, ln.n_scatter = static_cast<int>(wsc2.size());
+        ln.w_tree = b->w_tree, ln.n_tree = static_cast<int>(wtr.size());
+        ln.w_mark = b->w_mark, ln.n_mark = static_cast<int>(wmk.size());
+        ln.list = batch_list(b, of_lane[0]), ln.n_gather = static_cast<int>(std::min<int64_t>(kGatherBlocks, items));
+        break;
+      }
       for (size_t g = 0; g < blocks.size(); g++) {
         std::vector<Work> wl = mine(by_block[g]);
         if (wl.empty()) continue;
@@ -1615,24 +1772,42 @@ int batch_build(clay_batch* b) {
                              std::get<2>(blocks[g]) != 0});
         ln.n_part += static_cast<int>(wl.size());
       }
-      const std::vector<Work> le = mine(we), lsc = mine(wsc), lss = mine(wss), lsr = mine(wsr);
+      const std::vector<Work> le = mine(we), lsc = mine(wsc), lso = mine(wso), lsc2 = mine(wsc2), lss = mine(wss),
+                              lsr = mine(wsr), ltr = mine(wtr), lmk = mine(wmk);
       if ((rc = b->upload_table(&ln.w_emit, le)) || (rc = b->upload_table(&ln.w_scan, lsc)) ||
-          (rc = b->upload_table(&ln.w_ssplat, lss)) || (rc = b->upload_table(&ln.w_sres, lsr)))
+          (rc = b->upload_table(&ln.w_sort, lso)) ||
+          (rc = b->upload_table(&ln.w_scatter, lsc2)) || (rc = b->upload_table(&ln.w_ssplat, lss)) ||
+          (rc = b->upload_table(&ln.w_sres, lsr)) || (rc = b->upload_table(&ln.w_tree, ltr)) || (rc = b->upload_table(&ln.w_mark, lmk)))
         return rc;
       ln.n_emit = static_cast<int>(le.size());
       ln.n_scan = static_cast<int>(lsc.size());
+      ln.n_sort = static_cast<int>(lso.size());
+      ln.n_scatter = static_cast<int>(lsc2.size());
       ln.n_ssplat = static_cast<int>(lss.size());
       ln.n_sres = static_cast<int>(lsr.size());
+      ln.n_tree = static_cast<int>(ltr.size());
+      ln.n_mark = static_cast<int>(lmk.size());
+      int64_t mine_items = 0;
+      for (size_t i = 0; i < b->sims.size(); i++)
+        if (lane_of[i] == l && ss[i].gs) mine_items += b->sims[i]->surface->blocks();
+      ln.list = batch_list(b, of_lane[static_cast<size_t>(l)]);
+      ln.n_gather = static_cast<int>(std::min<int64_t>(kGatherBlocks, mine_items));
       if (l > 0 && !ln.stream) CK(cudaStreamCreateWithFlags(&ln.stream, cudaStreamNonBlocking));
       if (l > 0 && !ln.done) CK(cudaEventCreateWithFlags(&ln.done, cudaEventDisableTiming));
     }
   }
+  if ((rc = b->upload_staged())) return rc;
   b->n_emit = static_cast<int>(we.size());
   b->n_scan = static_cast<int>(wsc.size());
   b->n_xsplat = static_cast<int>(wxs.size());
   b->n_xres = static_cast<int>(wxr.size());
+  b->n_sort = static_cast<int>(wso.size());
+  b->n_scatter = static_cast<int>(wsc2.size());
   b->n_ssplat = static_cast<int>(wss.size());
   b->n_sres = static_cast<int>(wsr.size());
+  b->n_tree = static_cast<int>(wtr.size());
+  b->n_mark = static_cast<int>(wmk.size());
+  b->n_gather = static_cast<int>(std::min<int64_t>(kGatherBlocks, items));
   if (!b->side) CK(cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking));
   if (!b->ev_fork) CK(cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming));
   if (!b->ev_join) CK(cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming));
@@ -1689,6 +1864,16 @@ int batch_enqueue(clay_batch* b, cudaStream_t s) {
     if (!joined) CK(cudaStreamWaitEvent(ls, b->ev_join, 0));
     if (ln.n_ssplat) CK(L_splat(b->d_surf, ln.w_ssplat, ln.n_ssplat, 1, kSplatAccVoxels, ls));
     if (ln.n_sres) CK(L_resolve(b->d_surf, ln.w_sres, ln.n_sres, ls));
+    if (ln.n_sort) {
+      CK(L_sort_scan(d, b->d_surf, ln.w_sort, ln.n_sort, false, ls));
+      CK(L_sort_scan(d, b->d_surf, ln.w_sort, ln.n_sort, true, ls));
+      CK(L_sort_scatter(d, b->d_surf, ln.w_scatter, ln.n_scatter, ls));
+    }
+    if (ln.n_tree) {
+      CK(L_bake_tree(b->d_surf, ln.w_tree, ln.n_tree, ln.list, ls));
+      CK(L_bake_mark(b->d_surf, ln.w_mark, ln.n_mark, ln.list, ls));
+      CK(L_bake_gather(b->d_surf, ln.n_gather, ln.list, ls));
+    }
     if (li > 0) CK(cudaEventRecord(ln.done, ls));
   }
   for (size_t li = 1; li < b->lanes.size(); li++) CK(cudaStreamWaitEvent(s, b->lanes[li].done, 0));
@@ -1929,6 +2114,19 @@ int clay_batch_profile(clay_batch* b, void* stream, clay_phase_time* out, int ca
   }
   if (b->n_ssplat && (rc = timed("splat", [&] { return L_splat(b->d_surf, b->w_ssplat, b->n_ssplat, 1, kSplatAccVoxels, s); }))) return rc;
   if (b->n_sres && (rc = timed("resolve", [&] { return L_resolve(b->d_surf, b->w_sres, b->n_sres, s); }))) return rc;
+  if (b->n_sort) {
+    if ((rc = timed("bake_sort", [&] { return L_sort_scan(d, b->d_surf, b->w_sort, b->n_sort, false, s); }))) return rc;
+    if ((rc = timed("bake_sort", [&] { return L_sort_scan(d, b->d_surf, b->w_sort, b->n_sort, true, s); }))) return rc;
+    if ((rc = timed("bake_scatter", [&] { return L_sort_scatter(d, b->d_surf, b->w_scatter, b->n_scatter, s); }))) return rc;
+  }
+  if (b->n_tree) {
+    std::vector<int> all(b->sims.size());
+    for (size_t i = 0; i < all.size(); i++) all[i] = static_cast<int>(i);
+    const BakeList list = batch_list(b, all);
+    if ((rc = timed("bake_tree", [&] { return L_bake_tree(b->d_surf, b->w_tree, b->n_tree, list, s); }))) return rc;
+    if ((rc = timed("bake_mark", [&] { return L_bake_mark(b->d_surf, b->w_mark, b->n_mark, list, s); }))) return rc;
+    if ((rc = timed("bake_gather", [&] { return L_bake_gather(b->d_surf, b->n_gather, list, s); }))) return rc;
+  }
   CK(cudaStreamSynchronize(s));
   std::vector<clay_phase_time> agg;
   for (auto& r : recs) {
@@ -2023,23 +2221,31 @@ int clay_batch_step_subset(clay_batch* b, const int32_t* scenes, int n, void* st
     for (uint32_t p = 0; p < f->parts_scan; p++) tab.push_back({static_cast<uint32_t>(scenes[q]), p, 0u, 0u});
   }
   const int n_scan = mark() - o_scan;
-  const int o_splat = mark();
+  // the splat's tables, and the gather's for the scenes that the device may gather
+  std::vector<Work> splat, resolve, sort, scatter, tree, marks;
+  int64_t items = 0, particles = 0;
+  for (int q = 0; q < n; q++) particles += b->sims[scenes[q]]->live;
+  const BakeList list = batch_list(b, std::vector<int>(scenes, scenes + n));
+  const bool gather = b->gather && particles >= kGatherBatch && list.items;
   for (int q = 0; q < n; q++) {
     clay_fluid* f = b->sims[scenes[q]];
-    int64_t it = (f->substeps > 0 && f->live > 0) ? f->live : 0;
-    for (int m = 0; m < f->surface->mips; m++)
-      for (int64_t x = 0; x < it; x += kSplatThreads)
-        tab.push_back({static_cast<uint32_t>(scenes[q]), static_cast<uint32_t>(m), static_cast<uint32_t>(x),
-                       static_cast<uint32_t>(std::min<int64_t>(kSplatThreads, it - x))});
+    const int64_t it = (f->substeps > 0 && f->live > 0) ? f->live : 0;
+    add_splat_work(splat, resolve, static_cast<uint32_t>(scenes[q]), f->surface, it, kSplatThreads);
+    if (!gather || it < kGatherMin) continue;
+    add_bake_work(sort, scatter, tree, marks, static_cast<uint32_t>(scenes[q]), f->surface, it);
+    items += f->surface->blocks();
   }
-  const int n_splat = mark() - o_splat;
-  const int o_res = mark();
-  for (int q = 0; q < n; q++) {
-    int64_t quads = (b->sims[scenes[q]]->surface->vol->total + 3) / 4;
-    for (int64_t x = 0; x < quads; x += kResolveThreads)
-      tab.push_back({static_cast<uint32_t>(scenes[q]), 0u, static_cast<uint32_t>(x), kResolveThreads});
-  }
-  const int n_res = mark() - o_res;
+  auto place = [&](const std::vector<Work>& w, int& n_out) {
+    const int o = mark();
+    n_out = static_cast<int>(w.size());
+    tab.insert(tab.end(), w.begin(), w.end());
+    return o;
+  };
+  int n_splat = 0, n_res = 0, n_sort = 0, n_scatter = 0, n_tree = 0, n_mark = 0;
+  const int o_splat = place(splat, n_splat), o_res = place(resolve, n_res), o_sort = place(sort, n_sort),
+            o_scatter = place(scatter, n_scatter), o_tree = place(tree, n_tree), o_mark = place(marks, n_mark);
+  // a frame that gathers nothing takes the surfaces as plain splats
+  const SplatDev* surf = gather ? b->d_surf : b->d_surf_splat;
   // upload params + tables through double-buffered pinned memory
   int k = b->sub_slot;
   b->sub_slot ^= 1;
@@ -2088,8 +2294,18 @@ int clay_batch_step_subset(clay_batch* b, const int32_t* scenes, int n, void* st
       CK(L_forces_fast(d, W + o_part, n_part, T, sub, s));
     }
   }
-  if (n_splat) CK(L_splat(b->d_surf, W + o_splat, n_splat, 1, kSplatAccVoxels, s));
-  if (n_res) CK(L_resolve(b->d_surf, W + o_res, n_res, s));
+  if (n_splat) CK(L_splat(surf, W + o_splat, n_splat, 1, kSplatAccVoxels, s));
+  if (n_res) CK(L_resolve(surf, W + o_res, n_res, s));
+  if (n_sort) {
+    CK(L_sort_scan(d, surf, W + o_sort, n_sort, false, s));
+    CK(L_sort_scan(d, surf, W + o_sort, n_sort, true, s));
+    CK(L_sort_scatter(d, surf, W + o_scatter, n_scatter, s));
+  }
+  if (n_tree) {
+    CK(L_bake_tree(surf, W + o_tree, n_tree, list, s));
+    CK(L_bake_mark(surf, W + o_mark, n_mark, list, s));
+    CK(L_bake_gather(surf, static_cast<int>(std::min<int64_t>(kGatherBlocks, items)), list, s));
+  }
   return CLAY_OK;
 }
 

@@ -178,8 +178,52 @@ struct __align__(16) SplatDev {
   // of the particles' own boxes; the block walk is taken while its pairs (x2 for discs) are at
   // most walk_weight times those of the own boxes.
   uint32_t tile_ratio, walk_weight;
+  // A fluid's surface: its cell-build state, by which the device chooses between the splat and the
+  // gather (see bake_gathers). NULL: k_splat bakes the cloud, whatever it looks like.
+  const GridState* gs;
+  // The cloud's particles in bake order with their bounding boxes (see k_bake_tree), scratch of
+  // one gather.
+  float4* bpos;
+  float4 *leaf, *group, *super;
+  uint32_t* cursor;  // scratch of the bake order's sort; NULL: bake in cell order
 };
 constexpr uint32_t kSplatTileRatio = 6, kSplatWalkWeight = 3;
+
+// The box tree over a cloud in spatially coherent order: 32 particles per leaf, 32 leaves per
+// group, 32 groups per super-group, each box as two float4 (low, high corner).
+constexpr uint32_t kLeafN = 32, kGroupN = 32 * kLeafN, kSuperN = 32 * kGroupN;
+// Scratch of the tree of `n` particles, in 16-byte units, and where its parts start.
+struct BakeTreeLayout {
+  uint64_t leaf, group, super, cursor, list, total;
+};
+// A cloud may be gathered from kGatherMin particles on. A scene by itself is gathered from kGatherAlone on,
+// scenes of a batch when they hold kGatherBatch together: below, the gather's launches and the latency
+// of its descents cost more than the splat (4,096 particles alone: 167 us a frame with the splat, 171 with
+// the gather; five scenes of 36,000 together: 186 and 207).
+constexpr uint32_t kGatherMin = 64, kGatherAlone = 1u << 17, kGatherBatch = 1u << 18;
+// Scenes of more particles than kSortMin are baked in Morton order (see k_sort_scan): at most kSortBins
+// bins, scanned in parts.
+constexpr uint32_t kSortMin = 8192, kSortBins = 1u << 18, kSortPart = 2048, kSortParts = kSortBins / kSortPart + 1;
+__host__ __device__ inline BakeTreeLayout bake_tree_layout(uint64_t n) {
+  BakeTreeLayout l;
+  l.leaf = (n + kLeafN - 1) / kLeafN * kLeafN;  // the positions, padded to whole leaves
+  l.group = l.leaf + 2 * ((n + kLeafN - 1) / kLeafN);
+  l.super = l.group + 2 * ((n + kGroupN - 1) / kGroupN);
+  l.cursor = l.super + 2 * ((n + kSuperN - 1) / kSuperN);
+  l.list = l.cursor + (n > kSortMin ? (kSortBins + 1 + kSortParts + 3) / 4 : 0);
+  l.total = l.list;  // the list of a scene gathered by itself follows: see bake_list_fits
+  return l;
+}
+// The blocks of 8 x 4 x 2 voxels within reach of a cloud, as (object | level << 28, block index in
+// its level), from the front those taken eight voxels at a time, from the back the others; and the
+// counters: how many at the front, how many tickets the gather pass has drawn, how many at the back.
+struct BakeList {
+  uint2* items;
+  uint32_t* ctr;
+  uint32_t cap;
+};
+// Bytes of a list's counters, before its items.
+constexpr uint64_t kListCounterBytes = 16;
 
 // A unit of work of one launch: object index (scene or splat), sub-index (mip level or
 // scan part), first element, element count.
@@ -1316,6 +1360,19 @@ __device__ __forceinline__ uint32_t enc_key(float sd, float bw) {
   return static_cast<uint32_t>((v + 1.0f) * 32767.5f);
 }
 
+// Whether a fluid's surface is gathered: a voxel's descent costs about as much whatever the
+// cloud, a splat's particle costs the voxels of its band (splat.ts:238-246: 300 to 400 a level), so the
+// gather wins where particles are many for the voxels that they reach. They are where the occupied box is
+// densely filled, two a cell and more (1.4 M particles in 96 piles: 0.75 -> 0.35 ms), or where there is at
+// least one for eight voxels of the finest level, however they lie (262,144 as a thin spray into
+// 128^3: 0.61 -> 0.48 ms); a spray of 113,500 into 128^3 took 0.2 ms longer. gs == NULL: always splatted.
+__device__ __forceinline__ bool bake_gathers(const SplatDev& D) {
+  if (!D.gs) return false;
+  const uint64_t n = min(*D.live_count, D.capacity), r = static_cast<uint64_t>(D.r[0]);
+  const uint64_t cells = D.gs->L;
+  return n >= kGatherMin && ((cells > 0 && n >= 2 * cells) || 8 * n >= r * r * r);
+}
+
 __device__ __forceinline__ bool cloud_live(const SplatDev& D, uint32_t idx, uint32_t& i) {
   if (D.order) {
     uint32_t n = min(*D.live_count, D.capacity);
@@ -2159,12 +2216,533 @@ __global__ void __launch_bounds__(32 * kSplatWarps, 4) k_splat(const SplatDev* _
                                                              uint32_t acc_cap) {
   const Work w = get_work_reversed(work);
   const SplatDev& D = splats[w.obj];
+  if (bake_gathers(D)) return;
   splat_block(D, w, D.vp->origin[0], D.vp->origin[1], D.vp->origin[2], acc_cap);
 }
 
 __global__ void k_resolve(const SplatDev* __restrict__ splats, const Work* __restrict__ work) {
   const Work w = get_work(work);
+  if (bake_gathers(splats[w.obj])) return;
   resolve_block(splats[w.obj], w);
+}
+
+// ---------------------------------------------------------------------------------------
+// The bake as a gather: every voxel finds its nearest particle.
+//
+// A splat lowers each voxel by every particle whose band reaches it: a voxel in a dense fluid is
+// within the band of thousands of particles, of which one decides its value. Here a voxel keeps
+// its smallest squared length and descends a tree of bounding boxes over the cell-ordered cloud,
+// leaving out every box that is no nearer than that. The lengths are the splat's (the same f32
+// operations in the same order), a minimum does not depend on the order it is taken in, and a
+// box's own length bounds those of its particles exactly: rounding is monotone, so
+// fl(c - p) >= fl(c - hi) for p <= hi, and likewise through the squares and sums. The keys
+// are the reference's bit for bit.
+//
+// Three launches: k_bake_tree (positions in bake order and their boxes), k_bake_mark (voxels out of
+// reach of the cloud are written at once, the blocks within reach go to a list) and
+// k_bake_gather (the listed blocks).
+// The box of a warp's points (32 lanes), as order-preserving integers.
+__device__ __forceinline__ void warp_box(bool ok, float x, float y, float z, float4& lo, float4& hi) {
+  const uint32_t none_lo = sd_bits(__int_as_float(0x7f800000)), none_hi = sd_bits(-__int_as_float(0x7f800000));
+  lo = make_float4(bits_sd(__reduce_min_sync(0xffffffffu, ok ? sd_bits(x) : none_lo)),
+                   bits_sd(__reduce_min_sync(0xffffffffu, ok ? sd_bits(y) : none_lo)),
+                   bits_sd(__reduce_min_sync(0xffffffffu, ok ? sd_bits(z) : none_lo)), 0.0f);
+  hi = make_float4(bits_sd(__reduce_max_sync(0xffffffffu, ok ? sd_bits(x) : none_hi)),
+                   bits_sd(__reduce_max_sync(0xffffffffu, ok ? sd_bits(y) : none_hi)),
+                   bits_sd(__reduce_max_sync(0xffffffffu, ok ? sd_bits(z) : none_hi)), 0.0f);
+}
+
+// The bake order of a large scene. Cells along x are adjacent in the cell order, which makes
+// boxes of 32 consecutive particles long and thin where the fluid is sparse, and boxes of 1,024
+// long everywhere. So the cells' particles are put in Morton order of bins of (2^shift)^3
+// cells of the occupied box: the bins' sizes follow from the cell table, a scan in Morton order gives
+// their places, and the particles of a bin follow in any order.
+struct BakeBins {
+  uint32_t shift, kx, ky, kz, bins;  // bits per axis; `bins` in all, then one for the particles outside the grid
+};
+__device__ __forceinline__ BakeBins bake_bins(const BoxInfo& b, uint32_t n) {
+  BakeBins q;
+  const uint32_t most = min(kSortBins, n);
+  for (q.shift = 0;; q.shift++) {
+    auto bits = [&](uint32_t cells) { return cells > 1 ? 32u - __clz(((cells - 1) >> q.shift)) : 0u; };
+    q.kx = bits(b.bx);
+    q.ky = bits(b.by);
+    q.kz = bits(b.bz);
+    if (q.kx + q.ky + q.kz <= 18u && (1u << (q.kx + q.ky + q.kz)) <= most) break;
+  }
+  q.bins = b.L > 0 ? 1u << (q.kx + q.ky + q.kz) : 0u;
+  return q;
+}
+// Interleaves the bits of three bin coordinates, lowest first, as far as each axis has any.
+__device__ __forceinline__ uint32_t bin_code(const BakeBins& q, uint32_t x, uint32_t y, uint32_t z) {
+  uint32_t c = 0, o = 0;
+  for (uint32_t i = 0; i < max(q.kx, max(q.ky, q.kz)); i++) {
+    if (i < q.kx) c |= ((x >> i) & 1u) << o++;
+    if (i < q.ky) c |= ((y >> i) & 1u) << o++;
+    if (i < q.kz) c |= ((z >> i) & 1u) << o++;
+  }
+  return c;
+}
+// Particles in bin `code`: the cell table's ranges of its rows of cells.
+__device__ __forceinline__ uint32_t bin_size(const SceneDev& S, const BoxInfo& b, const BakeBins& q, uint32_t code) {
+  if (code == q.bins) return S.cell_start[b.L + 1] - S.cell_start[b.L];
+  uint32_t x = 0, y = 0, z = 0;
+  for (uint32_t i = 0; i < max(q.kx, max(q.ky, q.kz)); i++) {
+    if (i < q.kx) { x |= (code & 1u) << i; code >>= 1; }
+    if (i < q.ky) { y |= (code & 1u) << i; code >>= 1; }
+    if (i < q.kz) { z |= (code & 1u) << i; code >>= 1; }
+  }
+  const uint32_t side = 1u << q.shift, xa = x << q.shift, xb = min(xa + side, b.bx);
+  if (xa >= b.bx) return 0u;
+  uint32_t s = 0;
+  for (uint32_t cz = z << q.shift; cz < min((z + 1) << q.shift, b.bz); cz++)
+    for (uint32_t cy = y << q.shift; cy < min((y + 1) << q.shift, b.by); cy++) {
+      const uint32_t row = b.bx * (cy + b.by * cz);
+      s += S.cell_start[row + xb] - S.cell_start[row + xa];
+    }
+  return s;
+}
+
+// The bins' places, in two passes over parts of kSortPart bins (a block each): sums, then the scan.
+template <bool kFinal>
+__global__ void __launch_bounds__(1024) k_sort_scan(const SceneDev* __restrict__ scenes, const SplatDev* __restrict__ splats,
+                                                    const Work* __restrict__ work) {
+  Work w;
+  if (work) w = work[blockIdx.x];
+  else w = {0u, blockIdx.x, 0u, 0u};
+  const SceneDev& S = scenes[w.obj];
+  const SplatDev& D = splats[w.obj];
+  const uint32_t n = work_count(S);
+  if (!bake_gathers(D)) return;
+  const BoxInfo b = box_from_state(S.gs);
+  const BakeBins q = bake_bins(b, n);
+  const uint32_t beg = w.sub * kSortPart, end = min(beg + kSortPart, q.bins + 1u);
+  if (beg >= end) return;
+  uint32_t* __restrict__ part = D.cursor + kSortBins + 1u;
+  const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+  constexpr uint32_t kPer = kSortPart / 1024;
+  uint32_t size[kPer], sum = 0;
+#pragma unroll
+  for (uint32_t j = 0; j < kPer; j++) {
+    const uint32_t c = beg + threadIdx.x * kPer + j;
+    size[j] = c < end ? bin_size(S, b, q, c) : 0u;
+    sum += size[j];
+  }
+  __shared__ uint32_t s_w[32];
+  uint32_t x = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= static_cast<uint32_t>(o)) x += y;
+  }
+  if (lane == 31) s_w[wid] = x;
+  __syncthreads();
+  if constexpr (!kFinal) {
+    if (wid == 0) {
+      const uint32_t t = __reduce_add_sync(0xffffffffu, s_w[lane]);
+      if (lane == 0) part[w.sub] = t;
+    }
+  } else {
+    // what comes before: the earlier parts, the earlier warps, the earlier lanes
+    uint32_t before = __reduce_add_sync(0xffffffffu, lane < wid ? s_w[lane] : 0u);
+    for (uint32_t p0 = 0; p0 < w.sub; p0 += 32) before += __reduce_add_sync(0xffffffffu, p0 + lane < w.sub ? part[p0 + lane] : 0u);
+    uint32_t at = before + x - sum;
+#pragma unroll
+    for (uint32_t j = 0; j < kPer; j++) {
+      const uint32_t c = beg + threadIdx.x * kPer + j;
+      if (c < end) D.cursor[c] = at;
+      at += size[j];
+    }
+  }
+}
+
+// Positions relative to the volume origin, each to the next free place of its bin (one atomic per
+// bin and warp).
+__global__ void __launch_bounds__(256) k_sort_scatter(const SceneDev* __restrict__ scenes, const SplatDev* __restrict__ splats,
+                                                      const Work* __restrict__ work) {
+  const Work w = get_work(work);
+  const SceneDev& S = scenes[w.obj];
+  const SplatDev& D = splats[w.obj];
+  if (!bake_gathers(D)) return;
+  const uint32_t n = work_count(S), k = w.first + threadIdx.x, lane = threadIdx.x & 31u;
+  const bool act = k < n && threadIdx.x < w.n;
+  const BoxInfo b = box_from_state(S.gs);
+  const BakeBins q = bake_bins(b, max(n, 1u));
+  uint32_t code = 0xffffffffu;
+  float4 p = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (act) {
+    const uint32_t id = S.sorted_id[k], l = S.key[id];
+    p = S.parts[id].a;
+    code = l >= b.L ? q.bins
+                    : bin_code(q, (l % b.bx) >> q.shift, ((l / b.bx) % b.by) >> q.shift, (l / (b.bx * b.by)) >> q.shift);
+  }
+  const uint32_t peers = __match_any_sync(0xffffffffu, code);
+  if (!act) return;
+  const int leader = __ffs(peers) - 1;
+  uint32_t base = 0;
+  if (static_cast<int>(lane) == leader) base = atomicAdd(&D.cursor[code], static_cast<uint32_t>(__popc(peers)));
+  base = __shfl_sync(peers, base, leader);
+  D.bpos[base + __popc(peers & ((1u << lane) - 1u))] =
+      make_float4(p.x - D.vp->origin[0], p.y - D.vp->origin[1], p.z - D.vp->origin[2], 0.0f);
+}
+
+// Positions relative to the volume origin in bake order, leaf and group boxes: a block per group
+// of 1,024 particles. A position that is not a number lowers no voxel and enters no box.
+__global__ void __launch_bounds__(kGroupN) k_bake_tree(const SplatDev* __restrict__ splats, const Work* __restrict__ work,
+                                                       const BakeList list) {
+  const Work w = get_work(work);
+  const SplatDev& D = splats[w.obj];
+  if (blockIdx.x == 0 && threadIdx.x < 3) list.ctr[threadIdx.x] = 0u;
+  const uint32_t n = min(*D.live_count, D.capacity);
+  if (w.first >= n || !bake_gathers(D)) return;
+  __shared__ float4 s_lo[32], s_hi[32];
+  const uint32_t k = w.first + threadIdx.x, lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+  const float inf = __int_as_float(0x7f800000);
+  float px = inf, py = inf, pz = inf;
+  if (k < n && D.cursor) {  // k_sort_scatter put them in order
+    const float4 p = D.bpos[k];
+    px = p.x;
+    py = p.y;
+    pz = p.z;
+  } else if (k < n) {
+    const float4 p = *reinterpret_cast<const float4*>(D.pos + static_cast<size_t>(D.order[k]) * D.pos_stride);
+    px = p.x - D.vp->origin[0];
+    py = p.y - D.vp->origin[1];
+    pz = p.z - D.vp->origin[2];
+  }
+  const uint32_t leaf = k / kLeafN;
+  if (leaf * kLeafN < n) D.bpos[k] = make_float4(px, py, pz, 0.0f);
+  float4 lo, hi;
+  warp_box(k < n && px == px && py == py && pz == pz, px, py, pz, lo, hi);
+  if (lane == 0) {
+    s_lo[wid] = lo;
+    s_hi[wid] = hi;
+    if (leaf * kLeafN < n) {
+      D.leaf[2 * leaf] = lo;
+      D.leaf[2 * leaf + 1] = hi;
+    }
+  }
+  __syncthreads();
+  if (wid == 0) {
+    lo = s_lo[lane];
+    hi = s_hi[lane];
+    float4 l2, h2, unused;
+    warp_box(true, lo.x, lo.y, lo.z, l2, unused);
+    warp_box(true, hi.x, hi.y, hi.z, unused, h2);
+    if (lane == 0) {
+      D.group[2 * (w.first / kGroupN)] = l2;
+      D.group[2 * (w.first / kGroupN) + 1] = h2;
+    }
+  }
+}
+
+// key -> f16, as resolve[m] stores it (splat.ts:258-276).
+__device__ __forceinline__ __half key_half(uint32_t key) {
+  return __float2half_rn(static_cast<float>(key) * 3.0518043793392844e-05f - 1.0f);  // f32(1/32767.5)
+}
+
+// Squared length beyond which no particle can pass sd < bandWorld (a bound: the key decides).
+__device__ __forceinline__ float bake_reach2(float bw, float radius) { return (bw + radius) * (bw + radius) * 1.00001f; }
+
+// The row of 8 voxels at (x, y, z) of a level, out of reach.
+__device__ __forceinline__ void bake_fill_row(const SplatDev& D, long long v) {
+  const __half one = key_half(65535u);
+  const uint32_t h = __half_as_ushort(one), hh = h | (h << 16);
+  *reinterpret_cast<uint4*>(D.dist_out + v) = make_uint4(hh, hh, hh, hh);
+  if (D.key_capture) {
+    uint4* kc = reinterpret_cast<uint4*>(D.key_capture + v);
+    kc[0] = kc[1] = make_uint4(65535u, 65535u, 65535u, 65535u);
+  }
+}
+
+// A warp per chunk of 8^3 voxels (w.first: the first of the block's chunks, counted over all
+// levels): tests it against the group boxes, then its eight blocks of 8 x 4 x 2 voxels.
+constexpr int kMarkWarps = 8;
+// A block is taken eight voxels at a time where the voxels lie closer than this fraction of the
+// nearest group's extent.
+constexpr float kBrickExtent = 0.22f;
+__global__ void __launch_bounds__(32 * kMarkWarps) k_bake_mark(const SplatDev* __restrict__ splats, const Work* __restrict__ work,
+                                                               const BakeList list) {
+  Work w;
+  if (work) w = work[blockIdx.x];
+  else w = {0u, 0u, blockIdx.x * kMarkWarps, static_cast<uint32_t>(kMarkWarps)};
+  const SplatDev& D = splats[w.obj];
+  if (!bake_gathers(D)) return;
+  const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+  const uint32_t n = min(*D.live_count, D.capacity);
+  const uint32_t ng = (n + kGroupN - 1) / kGroupN;
+  uint32_t c = w.first + wid;
+  int m = 0;
+  uint32_t t = static_cast<uint32_t>(D.r[0]) >> 3;
+  uint32_t all = 0;
+  for (int l = 0; l < D.mips; l++) {
+    const uint32_t q = static_cast<uint32_t>(D.r[l]) >> 3;
+    all += q * q * q;
+  }
+  // super-group boxes for the gather pass, spread over the object's warps
+  for (uint32_t s = c; s * kSuperN < n; s += all) {
+    const uint32_t g = 32u * s + lane;
+    const float inf = __int_as_float(0x7f800000);
+    const float4 glo = g < ng ? D.group[2 * g] : make_float4(inf, inf, inf, 0.0f);
+    const float4 ghi = g < ng ? D.group[2 * g + 1] : make_float4(-inf, -inf, -inf, 0.0f);
+    float4 l2, h2, unused;
+    warp_box(true, glo.x, glo.y, glo.z, l2, unused);
+    warp_box(true, ghi.x, ghi.y, ghi.z, unused, h2);
+    if (lane == 0) {
+      D.super[2 * s] = l2;
+      D.super[2 * s + 1] = h2;
+    }
+  }
+  uint32_t near = 0;  // the chunk's blocks within reach
+  uint32_t closest = 0xffffffffu;  // squared length to the nearest group, and that group's largest extent
+  float extent = 0.0f;
+  bool in = c < all, brick = false;
+  uint32_t cx = 0, cy = 0, cz = 0;
+  if (in) {
+    while (c >= t * t * t) {
+      c -= t * t * t;
+      m++;
+      t = static_cast<uint32_t>(D.r[m]) >> 3;
+    }
+    cx = c % t;
+    cy = (c / t) % t;
+    cz = c / (t * t);
+    const float vx = D.voxel[m], reach2 = bake_reach2(D.bw[m], D.radius);
+    auto at = [&](uint32_t v) { return (static_cast<float>(v) + 0.5f) * vx; };
+    const float x0 = at(8 * cx), x1 = at(8 * cx + 7);
+    for (uint32_t g0 = 0; g0 < ng; g0 += 32) {
+      const uint32_t g = g0 + lane;
+      const float inf = __int_as_float(0x7f800000);
+      const float4 lo = g < ng ? D.group[2 * g] : make_float4(inf, inf, inf, 0.0f);
+      const float4 hi = g < ng ? D.group[2 * g + 1] : make_float4(-inf, -inf, -inf, 0.0f);
+      const float ex = fmaxf(fmaxf(lo.x - x1, x0 - hi.x), 0.0f);
+      auto reaches = [&](uint32_t ya, uint32_t yb, uint32_t za, uint32_t zb) {
+        const float ey = fmaxf(fmaxf(lo.y - at(yb), at(ya) - hi.y), 0.0f);
+        const float ez = fmaxf(fmaxf(lo.z - at(zb), at(za) - hi.z), 0.0f);
+        return (ex * ex + ey * ey) + ez * ez < reach2;
+      };
+      if (!__any_sync(0xffffffffu, reaches(8 * cy, 8 * cy + 7, 8 * cz, 8 * cz + 7))) continue;
+      {
+        const float ey = fmaxf(fmaxf(lo.y - at(8 * cy + 7), at(8 * cy) - hi.y), 0.0f);
+        const float ez = fmaxf(fmaxf(lo.z - at(8 * cz + 7), at(8 * cz) - hi.z), 0.0f);
+        const uint32_t d = __float_as_uint((ex * ex + ey * ey) + ez * ez), mn = __reduce_min_sync(0xffffffffu, d);
+        if (mn < closest) {
+          closest = mn;
+          extent = __shfl_sync(0xffffffffu, fmaxf(hi.x - lo.x, fmaxf(hi.y - lo.y, hi.z - lo.z)),
+                               __ffs(__ballot_sync(0xffffffffu, d == mn)) - 1);
+        }
+      }
+      for (uint32_t j = 0; j < 8; j++) {
+        const uint32_t ya = 8 * cy + 4 * (j & 1), za = 8 * cz + 2 * (j >> 1);
+        if (__any_sync(0xffffffffu, reaches(ya, ya + 3, za, za + 1))) near |= 1u << j;
+      }
+      if (near == 255u) break;
+    }
+    brick = vx < kBrickExtent * extent;
+  }
+  // one atomic per block of warps and way
+  __shared__ uint32_t s_cnt[2][kMarkWarps];
+  __shared__ uint32_t s_base[2];
+  if (lane < 2) s_cnt[lane][wid] = (lane == 0) == brick ? __popc(near) : 0u;
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    uint32_t sum = 0;
+    for (int k = 0; k < kMarkWarps; k++) {
+      const uint32_t q = s_cnt[threadIdx.x][k];
+      s_cnt[threadIdx.x][k] = sum;
+      sum += q;
+    }
+    s_base[threadIdx.x] = sum ? atomicAdd(&list.ctr[2 * threadIdx.x], sum) : 0u;
+  }
+  __syncthreads();
+  if (!in) return;
+  const uint32_t R = 8u * t;
+  if (lane < 8 && ((near >> lane) & 1u)) {
+    const uint32_t yy = 2 * cy + (lane & 1u), zz = 4 * cz + (lane >> 1);
+    const uint32_t way = brick ? 0u : 1u;
+    const uint32_t i = s_base[way] + s_cnt[way][wid] + __popc(near & ((1u << lane) - 1u));
+    list.items[brick ? i : list.cap - 1u - i] =
+        make_uint2(w.obj | (static_cast<uint32_t>(m) << 28), (zz * (2u * t) + yy) * t + cx);
+  }
+  for (uint32_t row = lane; row < 64; row += 32) {
+    const uint32_t y = row & 7u, z = row >> 3;
+    if ((near >> ((y >> 2) + 2 * (z >> 1))) & 1u) continue;
+    bake_fill_row(D, D.off[m] + 8ll * cx + static_cast<long long>(R) * ((8ll * cy + y) + static_cast<long long>(R) * (8ll * cz + z)));
+  }
+}
+
+// Squared length between two boxes (a point: both corners alike), in the operations and order of a
+// particle's; beyond every length where there is no node i.
+__device__ __forceinline__ uint32_t box_bits(const float4* __restrict__ nodes, uint32_t i, uint32_t n, float x0, float y0, float z0,
+                                             float x1, float y1, float z1) {
+  if (i >= n) return 0xffffffffu;
+  const float4 lo = nodes[2 * i], hi = nodes[2 * i + 1];
+  const float ex = fmaxf(fmaxf(lo.x - x1, x0 - hi.x), 0.0f);
+  const float ey = fmaxf(fmaxf(lo.y - y1, y0 - hi.y), 0.0f);
+  const float ez = fmaxf(fmaxf(lo.z - z1, z0 - hi.z), 0.0f);
+  return __float_as_uint((ex * ex + ey * ey) + ez * ez);
+}
+
+// A cloud's tree as a warp descends it: its lanes test the 32 boxes of a node at once against
+// a box (a voxel, or a warp's voxels), and go down into the nearest first, while it is nearer than
+// `best` (the largest of the squared lengths still to be lowered, the same in all lanes).
+struct BakeTree {
+  const float4* __restrict__ bpos;
+  const float4* __restrict__ leaf;
+  const float4* __restrict__ group;
+  const float4* __restrict__ super;
+  uint32_t n;
+  __device__ __forceinline__ explicit BakeTree(const SplatDev& D)
+      : bpos(D.bpos), leaf(D.leaf), group(D.group), super(D.super), n(min(*D.live_count, D.capacity)) {}
+
+  template <class F>
+  __device__ __forceinline__ void each_nearest(uint32_t d, const uint32_t& best, F&& visit) const {
+    for (;;) {
+      const uint32_t mn = __reduce_min_sync(0xffffffffu, d);
+      if (mn >= best) break;
+      const uint32_t k = static_cast<uint32_t>(__ffs(__ballot_sync(0xffffffffu, d == mn)) - 1);
+      if ((threadIdx.x & 31u) == k) d = 0xffffffffu;
+      visit(k);
+    }
+  }
+  // `wants(nodes, i)`: whether box i of a level is to be gone into after all.
+  template <class W, class F>
+  __device__ __forceinline__ void descend(float x0, float y0, float z0, float x1, float y1, float z1, const uint32_t& best,
+                                          W&& wants, F&& visit) const {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t nl = (n + kLeafN - 1) / kLeafN, ng = (n + kGroupN - 1) / kGroupN, ns = (n + kSuperN - 1) / kSuperN;
+    auto groups = [&](uint32_t s) {
+      each_nearest(box_bits(group, 32 * s + lane, ng, x0, y0, z0, x1, y1, z1), best, [&](uint32_t g) {
+        if (!wants(group, 32 * s + g)) return;
+        const uint32_t l0 = 32 * (32 * s + g);
+        each_nearest(box_bits(leaf, l0 + lane, nl, x0, y0, z0, x1, y1, z1), best, [&](uint32_t l) {
+          if (wants(leaf, l0 + l)) visit(l0 + l);
+        });
+      });
+    };
+    if (ns <= 1) {
+      groups(0);
+    } else {
+      for (uint32_t s0 = 0; s0 < ns; s0 += 32)
+        each_nearest(box_bits(super, s0 + lane, ns, x0, y0, z0, x1, y1, z1), best, [&](uint32_t s) { groups(s0 + s); });
+    }
+  }
+  // Lowers `best` to the nearest particle of one point, a leaf's particles a lane each;
+  // `lowered(p, k)`: lane k's particle p did.
+  template <class F>
+  __device__ __forceinline__ void nearest(float cx, float cy, float cz, uint32_t& best, F&& lowered) const {
+    descend(cx, cy, cz, cx, cy, cz, best, [](const float4*, uint32_t) { return true; }, [&](uint32_t l) {
+      const float4 p = bpos[l * kLeafN + (threadIdx.x & 31u)];
+      const float dx = cx - p.x, dy = cy - p.y, dz = cz - p.z;
+      const uint32_t d = __float_as_uint((dx * dx + dy * dy) + dz * dz), mn = __reduce_min_sync(0xffffffffu, d);
+      if (mn < best) {
+        best = mn;
+        lowered(p, __ffs(__ballot_sync(0xffffffffu, d == mn)) - 1);
+      }
+    });
+  }
+};
+
+__device__ __forceinline__ void bake_store(const SplatDev& D, int m, uint32_t x, uint32_t y, uint32_t z, uint32_t best) {
+  const long long R = D.r[m], v = D.off[m] + x + R * (y + R * static_cast<long long>(z));
+  const float bw = D.bw[m];
+  uint32_t key = 65535u;
+  if (best < 0x7f800000u) {
+    const float sd = __fsqrt_rn(__uint_as_float(best)) - D.radius;
+    if (sd < bw) key = enc_key(sd, bw);
+  }
+  D.dist_out[v] = key_half(key);
+  if (D.key_capture) D.key_capture[v] = key;
+}
+
+// The listed blocks of 8 x 4 x 2 voxels, in one of two ways (k_bake_mark chooses per block):
+//  - a warp per brick of 2^3 voxels: in a leaf, four particles against the eight voxels, eight times.
+//    The voxels share the way down and the leaves; good while leaves are about as large as the
+//    brick, so that its voxels need the same ones.
+//  - a warp per voxel, `run` voxels along x one after another: a leaf's 32 particles are read at
+//    once, a lane each, and the nearest particle of a voxel is the first guess of the next. Good where
+//    voxels are far apart for the cloud, and where the list is too short to fill the device.
+// Warps draw bricks, then runs.
+constexpr int kGatherWarps = 8;
+__global__ void __launch_bounds__(32 * kGatherWarps, 5) k_bake_gather(const SplatDev* __restrict__ splats, const BakeList list) {
+  const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * kGatherWarps;
+  const uint32_t near = list.ctr[0], wide = list.ctr[2], none = 0xffffffffu;
+  // too few blocks for a warp per eight voxels: all of them voxel by voxel
+  const uint32_t bricks = 8u * near >= warps ? 8u * near : 0u;
+  const uint32_t alone = bricks ? wide : near + wide;
+  uint32_t run_log = 3;  // shorter runs while there are fewer than four for each warp
+  while (run_log > 0 && (alone << (6 - run_log)) < 4u * warps) run_log--;
+  const uint32_t run = 1u << run_log, total = bricks + (alone << (6 - run_log));
+  // the first ticket is the warp's number, the next is drawn while one is being worked on
+  uint32_t ticket = blockIdx.x * kGatherWarps + (threadIdx.x >> 5), next = 0;
+  for (; ticket < total; ticket = __shfl_sync(0xffffffffu, next, 0)) {
+    if (lane == 0) next = warps + atomicAdd(&list.ctr[1], 1u);
+    const bool brick = ticket < bricks;
+    const uint32_t q = brick ? ticket >> 3 : (ticket - bricks) >> (6 - run_log);
+    const uint32_t q0 = brick ? ticket & 7u : ((ticket - bricks) << run_log) & 63u;  // the brick, or the run's first voxel
+    // the blocks taken brick by brick lie at the front of the list, the others at its back
+    const bool front = brick || (!bricks && q < near);
+    const uint2 it = list.items[front ? q : list.cap - 1u - (bricks ? q : q - near)];
+    const SplatDev& D = splats[it.x & 0x0fffffffu];
+    const int m = static_cast<int>(it.x >> 28);
+    const uint32_t R = static_cast<uint32_t>(D.r[m]), tx = R >> 3, ty = R >> 2;
+    const uint32_t bx = 8u * (it.y % tx), by = 4u * ((it.y / tx) % ty), bz = 2u * (it.y / (tx * ty));
+    const float voxel = D.voxel[m];
+    const uint32_t far = __float_as_uint(bake_reach2(D.bw[m], D.radius));
+    const BakeTree tree(D);
+    auto at = [&](uint32_t k) { return (static_cast<float>(k) + 0.5f) * voxel; };
+    if (brick) {
+      const uint32_t x0 = bx + 2u * (q0 & 3u), y0 = by + 2u * (q0 >> 2);
+      const uint32_t x = x0 + (lane & 1u), y = y0 + ((lane >> 1) & 1u), z = bz + ((lane >> 2) & 1u);
+      const float cx = at(x), cy = at(y), cz = at(z);
+      // `most`: the largest of the voxels' lengths so far, of those that have one
+      uint32_t best = far, most = far, least = far;
+      // a box that is within `most` of the brick may be too far for each of its voxels
+      auto wants = [&](const float4* __restrict__ nodes, uint32_t i) {
+        return __any_sync(0xffffffffu, box_bits(nodes, i, none, cx, cy, cz, cx, cy, cz) < best);
+      };
+      tree.descend(at(x0), at(y0), at(bz), at(x0 + 1), at(y0 + 1), at(bz + 1), most, wants, [&](uint32_t l) {
+        const float4* __restrict__ p = tree.bpos + (l * kLeafN + (lane >> 3));
+#pragma unroll
+        for (uint32_t j = 0; j < kLeafN; j += 8) {
+          const float4 a = p[j], b = p[j + 4];
+          const float ax = cx - a.x, ay = cy - a.y, az = cz - a.z, ux = cx - b.x, uy = cy - b.y, uz = cz - b.z;
+          best = __vimin3_u32(best, __float_as_uint((ax * ax + ay * ay) + az * az), __float_as_uint((ux * ux + uy * uy) + uz * uz));
+        }
+        best = min(best, __shfl_xor_sync(0xffffffffu, best, 8));
+        best = min(best, __shfl_xor_sync(0xffffffffu, best, 16));
+        const uint32_t reached = __reduce_max_sync(0xffffffffu, best < far ? best : 0u);
+        if (reached) most = reached, least = min(least, most);
+      });
+      // what was left out was at least `least` away from all of them: the voxels that have something
+      // nearer are done, the others (at the edge of the band) go down by themselves
+      for (uint32_t rest = __ballot_sync(0xffffffffu, best > least) & 255u; rest; rest &= rest - 1u) {
+        const int k = __ffs(rest) - 1;
+        const float sx = __shfl_sync(0xffffffffu, cx, k), sy = __shfl_sync(0xffffffffu, cy, k), sz = __shfl_sync(0xffffffffu, cz, k);
+        uint32_t b = __shfl_sync(0xffffffffu, best, k);
+        tree.nearest(sx, sy, sz, b, [](const float4&, int) {});
+        if (static_cast<int>(lane) == k) best = b;
+      }
+      if (lane < 8) bake_store(D, m, x, y, z, best);
+    } else {
+      const uint32_t x0 = bx + (q0 & 7u), y = by + ((q0 >> 3) & 3u), z = bz + (q0 >> 5);
+      const float cy = at(y), cz = at(z);
+      uint32_t mine = kNoHit;
+      float gx = __int_as_float(0x7f800000), gy = gx, gz = gx;  // the nearest particle so far
+      for (uint32_t x = 0; x < run; x++) {
+        const float cx = at(x0 + x);
+        const float hx = cx - gx, hy = cy - gy, hz = cz - gz;
+        uint32_t best = min(far, __float_as_uint((hx * hx + hy * hy) + hz * hz));
+        tree.nearest(cx, cy, cz, best, [&](const float4& p, int k) {
+          gx = __shfl_sync(0xffffffffu, p.x, k);
+          gy = __shfl_sync(0xffffffffu, p.y, k);
+          gz = __shfl_sync(0xffffffffu, p.z, k);
+        });
+        if (lane == x) mine = best;
+      }
+      if (lane < run) bake_store(D, m, x0 + lane, y, z, mine);
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------------------

@@ -83,6 +83,22 @@ cudaError_t L_splat(const SplatDev* d, const Work* w, int blocks, int blocks_y, 
   count_launch();
   return cudaPeekAtLastError();
 }
+cudaError_t L_sort_scan(const SceneDev* s, const SplatDev* d, const Work* w, int blocks, bool final, cudaStream_t st) {
+  if (final) CLAY_LAUNCH(k_sort_scan<true>, blocks, 1024, st, s, d, w);
+  CLAY_LAUNCH(k_sort_scan<false>, blocks, 1024, st, s, d, w);
+}
+cudaError_t L_sort_scatter(const SceneDev* s, const SplatDev* d, const Work* w, int blocks, cudaStream_t st) {
+  CLAY_LAUNCH(k_sort_scatter, blocks, 256, st, s, d, w);
+}
+cudaError_t L_bake_tree(const SplatDev* d, const Work* w, int blocks, BakeList list, cudaStream_t st) {
+  CLAY_LAUNCH(k_bake_tree, blocks, kGroupN, st, d, w, list);
+}
+cudaError_t L_bake_mark(const SplatDev* d, const Work* w, int blocks, BakeList list, cudaStream_t st) {
+  CLAY_LAUNCH(k_bake_mark, blocks, 32 * kMarkWarps, st, d, w, list);
+}
+cudaError_t L_bake_gather(const SplatDev* d, int blocks, BakeList list, cudaStream_t st) {
+  CLAY_LAUNCH(k_bake_gather, blocks, 32 * kGatherWarps, st, d, list);
+}
 cudaError_t L_resolve(const SplatDev* d, const Work* w, int blocks, cudaStream_t st) {
   CLAY_LAUNCH(k_resolve, blocks, kResolveThreads, st, d, w);
 }

@@ -46,6 +46,14 @@ cudaError_t L_forces_fast(const SceneDev* s, const Work* w, int blocks, int thre
 // acc_voxels: size of the shared-memory minimum tile (dynamic shared memory, 4 B per voxel).
 cudaError_t L_splat(const SplatDev* d, const Work* w, int blocks, int blocks_y, uint32_t acc_voxels, cudaStream_t st);
 cudaError_t L_resolve(const SplatDev* d, const Work* w, int blocks, cudaStream_t st);
+// The bake order of large scenes: parts of kSortPart bins, then blocks of 256 particles.
+cudaError_t L_sort_scan(const SceneDev* s, const SplatDev* d, const Work* w, int blocks, bool final, cudaStream_t st);
+cudaError_t L_sort_scatter(const SceneDev* s, const SplatDev* d, const Work* w, int blocks, cudaStream_t st);
+// The gather bake: `blocks` groups of 1,024 particles; blocks of kMarkChunks 8^3-voxel chunks over
+// all levels; and as many blocks as can work at once.
+cudaError_t L_bake_tree(const SplatDev* d, const Work* w, int blocks, BakeList list, cudaStream_t st);
+cudaError_t L_bake_mark(const SplatDev* d, const Work* w, int blocks, BakeList list, cudaStream_t st);
+cudaError_t L_bake_gather(const SplatDev* d, int blocks, BakeList list, cudaStream_t st);
 // SurfaceExtractor passes (grid passes: `blocks` blocks of kExtractThreads lattice cells).
 cudaError_t L_field_query_mip(const FieldDev* f, const float* pts, int n, int mip, float* sxy, float* fxy, cudaStream_t st);
 // ClaySolver passes.
@@ -73,5 +81,7 @@ cudaError_t L_field_query(const FieldDev* f, const float* pts, int n, float* sxy
 constexpr int kScanThreads = 1024;
 constexpr int kSplatThreads = 32 * kSplatWarps;
 constexpr int kResolveThreads = 256;
+constexpr int kMarkChunks = 8;         // 8^3-voxel chunks per block of the mark pass
+constexpr int kGatherBlocks = 148 * 5;  // the gather pass's blocks: what the device holds at once
 
 }  // namespace clay
