@@ -2610,7 +2610,7 @@ int clay_solver_step(clay_solver* sv, int32_t body_count, void* stream) {
     CK(L_pbd_kick(sv->d, blocks, s));
     sv->kicking = false;
   }
-  // The substeps' 4 x substeps dependent passes run as one CUDA graph, captured on a private
+  // The substeps' 1 + 2 x substeps dependent passes run as one CUDA graph, captured on a private
   // stream the first time and again when the body count changes.
   if (!sv->graph || sv->graph_bodies != body_count) {
     if (sv->graph) cudaGraphExecDestroy(sv->graph);
@@ -2620,11 +2620,10 @@ int clay_solver_step(clay_solver* sv, int32_t body_count, void* stream) {
     CK(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
     const uint64_t before = launch_count();
     cudaError_t e = cudaSuccess;
+    e = L_pbd_move(sv->d, blocks, false, true, cs);
     for (int sub = 0; sub < sv->substeps && e == cudaSuccess; sub++) {
-      e = L_pbd_predict(sv->d, blocks, cs);
-      if (e == cudaSuccess) e = L_pbd_match(sv->d, body_count, cs);
-      if (e == cudaSuccess) e = L_pbd_apply(sv->d, blocks, cs);
-      if (e == cudaSuccess) e = L_pbd_finalize(sv->d, blocks, cs);
+      e = L_pbd_match(sv->d, body_count, cs);
+      if (e == cudaSuccess) e = L_pbd_move(sv->d, blocks, true, sub + 1 < sv->substeps, cs);
     }
     sv->launches = static_cast<int64_t>(launch_count() - before);
     cudaGraph_t g = nullptr;

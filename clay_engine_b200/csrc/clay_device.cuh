@@ -271,6 +271,7 @@ struct __align__(16) SolveDev {
 };
 constexpr int kSolveThreads = 64;    // particle passes (pbd.ts:10)
 constexpr int kSolveReduce = 256;    // threads per body in the match pass (pbd.ts:8)
+constexpr uint32_t kSolveBatch = 8;  // particles a thread of it loads at once
 constexpr uint32_t kBodyKinematic = 1u, kBodyWeightless = 2u;  // BodyFlags (particles.ts:38-43)
 
 // The brush record (brush.ts:52-78), 80 bytes.
@@ -3528,51 +3529,111 @@ __global__ void __launch_bounds__(kSolveThreads) k_pbd_kick(const SolveDev* __re
   }
 }
 
-// predict (pbd.ts:172-222): BDF2 predictor, then the world collision with positional friction.
-__global__ void __launch_bounds__(kSolveThreads) k_pbd_predict(const SolveDev* __restrict__ sd) {
+// The particle passes around the match: predict (pbd.ts:172-222: BDF2 predictor, world collision
+// with positional friction), apply (pbd.ts:299-340: the pull towards the matched shape, a final projection
+// out of the world, plasticity letting the rest shape follow) and finalize (pbd.ts:342-372: first-order
+// velocity, damping, speed cap). Each works on one particle's record alone, so a substep's
+// apply and finalize and the next one's predict are one pass over the records, which are read and
+// written once, 16 bytes at a time. Bound by the record traffic (L2 for a set of this size): as
+// passes of their own with 4-byte accesses at the record's 96-byte stride, 326,800 particles took 20 (predict)
+// + 15 (apply) + 17 us (finalize) a substep; a step of two substeps 127.5 us, now 81.9.
+template <bool kTail, bool kHead>
+__global__ void __launch_bounds__(kSolveThreads) k_pbd_move(const SolveDev* __restrict__ sd) {
   const SolveDev& S = *sd;
   const uint32_t i = blockIdx.x * kSolveThreads + threadIdx.x;
   if (i >= static_cast<uint32_t>(S.capacity)) return;
-  const uint32_t b = pbd_owner(S, i);
+  float4* __restrict__ rec = reinterpret_cast<float4*>(S.particles + static_cast<size_t>(i) * 96);
+  const float4 r0 = rec[0], r1 = rec[1], r2 = rec[2], r3 = rec[3];
+  // ownerOf (pbd.ts:126-142)
+  const uint32_t b = __float_as_uint(r0.w);
   if (b >= static_cast<uint32_t>(S.max_bodies)) return;
-  const uint32_t flags = pbd_flags(S, b);
+  const float4* __restrict__ body = reinterpret_cast<const float4*>(S.bodies + static_cast<size_t>(b) * 64);
+  const float4 b0 = body[0], b2 = body[2], b3 = body[3];
+  const uint32_t first = __float_as_uint(b0.w), count = __float_as_uint(b2.w), flags = __float_as_uint(b3.w);
+  if (i < first || i >= first + count) return;
   if (flags & kBodyKinematic) return;
-  float* p = reinterpret_cast<float*>(S.particles + static_cast<size_t>(i) * 96);
-  float acc[3];
-  for (int k = 0; k < 3; k++) {
-    acc[k] = (flags & kBodyWeightless) ? 0.0f : S.gravity[k];
-    if (b == S.push_body) acc[k] = acc[k] + S.push[k];
+  float p[3] = {r0.x, r0.y, r0.z}, prev[3] = {r1.x, r1.y, r1.z}, vel[3] = {r2.x, r2.y, r2.z}, vp[3] = {r3.x, r3.y, r3.z};
+  if constexpr (kTail) {
+    const float4 b1 = body[1], r4 = rec[4];
+    const Q4 rot = {b1.x, b1.y, b1.z, b1.w};
+    float tx, ty, tz;
+    quat_rotate(rot, r4.x - b2.x, r4.y - b2.y, r4.z - b2.z, tx, ty, tz);
+    const float target[3] = {b0.x + tx, b0.y + ty, b0.z + tz};
+    const float st = clampf(b3.x, 0.0f, 1.0f), om = 1.0f - st;
+    float q[3];
+    for (int k = 0; k < 3; k++) q[k] = p[k] * om + target[k] * st;  // mix(pos, target, st)
+    float sx, sy;
+    const int child = field_pick(S.world, q[0], q[1], q[2], sx, sy);
+    if (sx < S.radius) {
+      float nx, ny, nz;
+      field_normal(S.world, child, q[0], q[1], q[2], nx, ny, nz);
+      const float push = S.radius - sx;
+      q[0] = q[0] + nx * push;
+      q[1] = q[1] + ny * push;
+      q[2] = q[2] + nz * push;
+      prev[0] = prev[0] + nx * push;
+      prev[1] = prev[1] + ny * push;
+      prev[2] = prev[2] + nz * push;
+    }
+    for (int k = 0; k < 3; k++) p[k] = q[k];
+    if (b3.y > 0.0f) {
+      const Q4 cj = {-rot.x, -rot.y, -rot.z, rot.w};
+      float rx, ry, rz;
+      quat_rotate(cj, q[0] - b0.x, q[1] - b0.y, q[2] - b0.z, rx, ry, rz);
+      const float pl = clampf(b3.y, 0.0f, 1.0f), om2 = 1.0f - pl;
+      rec[4] = make_float4(r4.x * om2 + (rx + b2.x) * pl, r4.y * om2 + (ry + b2.y) * pl, r4.z * om2 + (rz + b2.z) * pl, r4.w);
+    }
+    const float ih = __fdiv_rn(1.0f, fmaxf(S.h, 1e-6f));
+    float v[3];
+    for (int k = 0; k < 3; k++) v[k] = ((p[k] - prev[k]) * ih) * S.damping;
+    const float speed = len3(v[0], v[1], v[2]);
+    if (speed > S.max_speed) {
+      const float sc = __fdiv_rn(S.max_speed, speed);
+      for (int k = 0; k < 3; k++) v[k] = v[k] * sc;
+    }
+    for (int k = 0; k < 3; k++) {
+      vp[k] = vel[k];
+      vel[k] = v[k];
+    }
+    rec[2] = make_float4(vel[0], vel[1], vel[2], r2.w);
+    rec[3] = make_float4(vp[0], vp[1], vp[2], r3.w);
   }
-  const float third = 0.3333333432674407958984375f;  // f32(1 / 3)
-  const float h23 = __fdiv_rn(2.0f * S.h, 3.0f);
-  float q[3];
-  for (int k = 0; k < 3; k++) {
-    const float vpred = (p[8 + k] * 4.0f - p[12 + k]) * third + acc[k] * h23;
-    q[k] = (p[k] * 4.0f - p[4 + k]) * third + vpred * h23;
+  if constexpr (kHead) {
+    float acc[3];
+    for (int k = 0; k < 3; k++) {
+      acc[k] = (flags & kBodyWeightless) ? 0.0f : S.gravity[k];
+      if (b == S.push_body) acc[k] = acc[k] + S.push[k];
+    }
+    const float third = 0.3333333432674407958984375f;  // f32(1 / 3)
+    const float h23 = __fdiv_rn(2.0f * S.h, 3.0f);
+    float q[3];
+    for (int k = 0; k < 3; k++) {
+      const float vpred = (vel[k] * 4.0f - vp[k]) * third + acc[k] * h23;
+      q[k] = (p[k] * 4.0f - prev[k]) * third + vpred * h23;
+    }
+    for (int k = 0; k < 3; k++) prev[k] = p[k];
+    float sx, sy;
+    const int child = field_pick(S.world, q[0], q[1], q[2], sx, sy);
+    if (sx < S.radius) {
+      float nx, ny, nz;
+      field_normal(S.world, child, q[0], q[1], q[2], nx, ny, nz);
+      const float push = S.radius - sx;
+      q[0] = q[0] + nx * push;
+      q[1] = q[1] + ny * push;
+      q[2] = q[2] + nz * push;
+      prev[0] = p[0] + nx * push;
+      prev[1] = p[1] + ny * push;
+      prev[2] = p[2] + nz * push;
+      const float dx = q[0] - p[0], dy = q[1] - p[1], dz = q[2] - p[2];
+      const float dn = dot3(dx, dy, dz, nx, ny, nz);
+      q[0] = q[0] - (dx - nx * dn) * S.friction;
+      q[1] = q[1] - (dy - ny * dn) * S.friction;
+      q[2] = q[2] - (dz - nz * dn) * S.friction;
+    }
+    for (int k = 0; k < 3; k++) p[k] = q[k];
   }
-  float prev[3] = {p[0], p[1], p[2]};
-  float sx, sy;
-  const int child = field_pick(S.world, q[0], q[1], q[2], sx, sy);
-  if (sx < S.radius) {
-    float nx, ny, nz;
-    field_normal(S.world, child, q[0], q[1], q[2], nx, ny, nz);
-    const float push = S.radius - sx;
-    q[0] = q[0] + nx * push;
-    q[1] = q[1] + ny * push;
-    q[2] = q[2] + nz * push;
-    prev[0] = p[0] + nx * push;
-    prev[1] = p[1] + ny * push;
-    prev[2] = p[2] + nz * push;
-    const float dx = q[0] - p[0], dy = q[1] - p[1], dz = q[2] - p[2];
-    const float dn = dot3(dx, dy, dz, nx, ny, nz);
-    q[0] = q[0] - (dx - nx * dn) * S.friction;
-    q[1] = q[1] - (dy - ny * dn) * S.friction;
-    q[2] = q[2] - (dz - nz * dn) * S.friction;
-  }
-  for (int k = 0; k < 3; k++) {
-    p[4 + k] = prev[k];
-    p[k] = q[k];
-  }
+  rec[0] = make_float4(p[0], p[1], p[2], r0.w);
+  rec[1] = make_float4(prev[0], prev[1], prev[2], r1.w);
 }
 
 // match (pbd.ts:224-297): per body, the current and rest centroids and the covariance
@@ -3587,20 +3648,47 @@ __global__ void __launch_bounds__(kSolveReduce) k_pbd_match(const SolveDev* __re
   const uint32_t live = first >= cap ? 0u : min(count, cap - first);
   __shared__ float g[kSolveReduce][9];
   auto reduce = [&]() {
-    for (uint32_t s = kSolveReduce / 2; s > 0; s >>= 1) {
+    for (uint32_t s = kSolveReduce / 2; s >= 32; s >>= 1) {
       if (li < s)
         for (int k = 0; k < 9; k++) g[li][k] = g[li][k] + g[li + s][k];
       __syncthreads();
     }
+    if (li < 32)
+      for (uint32_t s = 16; s > 0; s >>= 1) {
+        if (li < s)
+          for (int k = 0; k < 9; k++) g[li][k] = g[li][k] + g[li + s][k];
+        __syncwarp();
+      }
+    __syncthreads();
+  };
+  // A thread's particles in order, kSolveBatch of them loaded before any is added: one block per body
+  // leaves the device to few threads, each waiting on its loads (one at a time: 17.3 us for 86
+  // bodies of 3,800 particles).
+  auto each = [&](auto&& add) {
+    for (uint32_t t = li; t < live; t += kSolveBatch * kSolveReduce) {
+      float4 p[kSolveBatch], r[kSolveBatch];
+#pragma unroll
+      for (uint32_t u = 0; u < kSolveBatch; u++) {
+        if (t + u * kSolveReduce < live) {
+          const float4* rec = reinterpret_cast<const float4*>(S.particles + static_cast<size_t>(first + t + u * kSolveReduce) * 96);
+          p[u] = rec[0];
+          r[u] = rec[4];
+        }
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < kSolveBatch; u++)
+        if (t + u * kSolveReduce < live) add(p[u], r[u]);
+    }
   };
   float sp[3] = {0.0f, 0.0f, 0.0f}, sr[3] = {0.0f, 0.0f, 0.0f};
-  for (uint32_t t = li; t < live; t += kSolveReduce) {
-    const float* p = reinterpret_cast<const float*>(S.particles + static_cast<size_t>(first + t) * 96);
-    for (int k = 0; k < 3; k++) {
-      sp[k] = sp[k] + p[k];
-      sr[k] = sr[k] + p[16 + k];
-    }
-  }
+  each([&](const float4 p, const float4 r) {
+    sp[0] = sp[0] + p.x;
+    sp[1] = sp[1] + p.y;
+    sp[2] = sp[2] + p.z;
+    sr[0] = sr[0] + r.x;
+    sr[1] = sr[1] + r.y;
+    sr[2] = sr[2] + r.z;
+  });
   for (int k = 0; k < 3; k++) {
     g[li][k] = sp[k];
     g[li][3 + k] = sr[k];
@@ -3613,13 +3701,12 @@ __global__ void __launch_bounds__(kSolveReduce) k_pbd_match(const SolveDev* __re
   const float rcom[3] = {g[0][3] * inv, g[0][4] * inv, g[0][5] * inv};
   __syncthreads();
   float a[9] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-  for (uint32_t t = li; t < live; t += kSolveReduce) {
-    const float* p = reinterpret_cast<const float*>(S.particles + static_cast<size_t>(first + t) * 96);
-    const float pr[3] = {p[0] - com[0], p[1] - com[1], p[2] - com[2]};
-    const float rr[3] = {p[16] - rcom[0], p[17] - rcom[1], p[18] - rcom[2]};
+  each([&](const float4 p, const float4 r) {
+    const float pr[3] = {p.x - com[0], p.y - com[1], p.z - com[2]};
+    const float rr[3] = {r.x - rcom[0], r.y - rcom[1], r.z - rcom[2]};
     for (int c = 0; c < 3; c++)
       for (int k = 0; k < 3; k++) a[3 * c + k] = a[3 * c + k] + pr[k] * rr[c];
-  }
+  });
   for (int k = 0; k < 9; k++) g[li][k] = a[k];
   __syncthreads();
   reduce();
@@ -3639,75 +3726,6 @@ __global__ void __launch_bounds__(kSolveReduce) k_pbd_match(const SolveDev* __re
     f[5] = r.y;
     f[6] = r.z;
     f[7] = r.w;
-  }
-}
-
-// apply (pbd.ts:299-340): the pull towards the matched shape, a final projection out of the
-// world, and plasticity letting the rest shape follow.
-__global__ void __launch_bounds__(kSolveThreads) k_pbd_apply(const SolveDev* __restrict__ sd) {
-  const SolveDev& S = *sd;
-  const uint32_t i = blockIdx.x * kSolveThreads + threadIdx.x;
-  if (i >= static_cast<uint32_t>(S.capacity)) return;
-  const uint32_t b = pbd_owner(S, i);
-  if (b >= static_cast<uint32_t>(S.max_bodies)) return;
-  const float* bf = reinterpret_cast<const float*>(S.bodies + static_cast<size_t>(b) * 64);
-  const uint32_t flags = *reinterpret_cast<const uint32_t*>(bf + 15);
-  if (flags & kBodyKinematic) return;
-  float* p = reinterpret_cast<float*>(S.particles + static_cast<size_t>(i) * 96);
-  const Q4 rot = {bf[4], bf[5], bf[6], bf[7]};
-  float tx, ty, tz;
-  quat_rotate(rot, p[16] - bf[8], p[17] - bf[9], p[18] - bf[10], tx, ty, tz);
-  const float target[3] = {bf[0] + tx, bf[1] + ty, bf[2] + tz};
-  const float st = clampf(bf[12], 0.0f, 1.0f), om = 1.0f - st;
-  float q[3];
-  for (int k = 0; k < 3; k++) q[k] = p[k] * om + target[k] * st;  // mix(pos, target, st)
-  float sx, sy;
-  const int child = field_pick(S.world, q[0], q[1], q[2], sx, sy);
-  if (sx < S.radius) {
-    float nx, ny, nz;
-    field_normal(S.world, child, q[0], q[1], q[2], nx, ny, nz);
-    const float push = S.radius - sx;
-    q[0] = q[0] + nx * push;
-    q[1] = q[1] + ny * push;
-    q[2] = q[2] + nz * push;
-    p[4] = p[4] + nx * push;
-    p[5] = p[5] + ny * push;
-    p[6] = p[6] + nz * push;
-  }
-  const float r0[3] = {p[16], p[17], p[18]};
-  p[0] = q[0];
-  p[1] = q[1];
-  p[2] = q[2];
-  if (bf[13] > 0.0f) {
-    const Q4 cj = {-rot.x, -rot.y, -rot.z, rot.w};
-    float rx, ry, rz;
-    quat_rotate(cj, q[0] - bf[0], q[1] - bf[1], q[2] - bf[2], rx, ry, rz);
-    const float rest[3] = {rx + bf[8], ry + bf[9], rz + bf[10]};
-    const float pl = clampf(bf[13], 0.0f, 1.0f), om2 = 1.0f - pl;
-    for (int k = 0; k < 3; k++) p[16 + k] = r0[k] * om2 + rest[k] * pl;
-  }
-}
-
-// finalize (pbd.ts:342-372): first-order velocity from the positions, damping, speed cap.
-__global__ void __launch_bounds__(kSolveThreads) k_pbd_finalize(const SolveDev* __restrict__ sd) {
-  const SolveDev& S = *sd;
-  const uint32_t i = blockIdx.x * kSolveThreads + threadIdx.x;
-  if (i >= static_cast<uint32_t>(S.capacity)) return;
-  const uint32_t b = pbd_owner(S, i);
-  if (b >= static_cast<uint32_t>(S.max_bodies)) return;
-  if (pbd_flags(S, b) & kBodyKinematic) return;
-  float* p = reinterpret_cast<float*>(S.particles + static_cast<size_t>(i) * 96);
-  const float ih = __fdiv_rn(1.0f, fmaxf(S.h, 1e-6f));
-  float v[3];
-  for (int k = 0; k < 3; k++) v[k] = ((p[k] - p[4 + k]) * ih) * S.damping;
-  const float speed = len3(v[0], v[1], v[2]);
-  if (speed > S.max_speed) {
-    const float sc = __fdiv_rn(S.max_speed, speed);
-    for (int k = 0; k < 3; k++) v[k] = v[k] * sc;
-  }
-  for (int k = 0; k < 3; k++) {
-    p[12 + k] = p[8 + k];
-    p[8 + k] = v[k];
   }
 }
 

@@ -58,10 +58,9 @@ cudaError_t L_bake_gather(const SplatDev* d, int blocks, BakeList list, cudaStre
 cudaError_t L_field_query_mip(const FieldDev* f, const float* pts, int n, int mip, float* sxy, float* fxy, cudaStream_t st);
 // ClaySolver passes.
 cudaError_t L_pbd_kick(const SolveDev* s, int blocks, cudaStream_t st);
-cudaError_t L_pbd_predict(const SolveDev* s, int blocks, cudaStream_t st);
 cudaError_t L_pbd_match(const SolveDev* s, int bodies, cudaStream_t st);
-cudaError_t L_pbd_apply(const SolveDev* s, int blocks, cudaStream_t st);
-cudaError_t L_pbd_finalize(const SolveDev* s, int blocks, cudaStream_t st);
+// The particle passes between two matches: `tail`: apply and finalize, `head`: the next predict.
+cudaError_t L_pbd_move(const SolveDev* s, int blocks, bool tail, bool head, cudaStream_t st);
 cudaError_t L_ext_reset(const ExtractDev* e, cudaStream_t st);
 cudaError_t L_ext_cells(const ExtractDev* e, int blocks, cudaStream_t st);
 cudaError_t L_ext_scan(const ExtractDev* e, int which, cudaStream_t st);
