@@ -64,6 +64,7 @@ namespace {
   } while (0)
 
 constexpr int TILE = 8;
+constexpr int kMaxBrushes = 256;  // one per thread of the build's cull
 constexpr int kMaxResolution = 4096;  // 4096^3 voxels per level: far beyond device memory, far below int64 overflow
 
 // SplatField's default mip count, Math.max(1, Math.log2(res / TILE) | 0) (splat.ts:149):
@@ -157,6 +158,7 @@ struct clay_volume {
   int total_cells = 0;
   __half* dist = nullptr;
   __half* mat = nullptr;
+  BrushDev* brushes = nullptr;  // of the last build
   VolParamsDev h{};
   VolParamsDev* d = nullptr;
   bool dirty = true;
@@ -428,6 +430,7 @@ void free_volume(clay_volume* v) {
   v->ctx->dev_free(v->dist, sizeof(__half) * v->total);
   v->ctx->dev_free(v->mat, sizeof(__half) * v->total);
   v->ctx->dev_free(v->d, sizeof(VolParamsDev));
+  v->ctx->dev_free(v->brushes, sizeof(BrushDev) * kMaxBrushes);
   delete v;
 }
 
@@ -749,22 +752,28 @@ int clay_volume_build_brushes(clay_volume* v, const clay_brush* brushes, int cou
   if (!v) return fail(CLAY_EINVAL, "clay_volume_build_brushes: NULL volume");
   if (count < 0 || (count > 0 && !brushes)) return fail(CLAY_EINVAL, "clay_volume_build_brushes: bad brush list");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  int n = std::min(count, 256);  // builder.ts:57,148-153
-  BrushDev* db = nullptr;
-  void* p = nullptr;
-  int rc = v->ctx->dev_alloc(&p, sizeof(BrushDev) * std::max(n, 1));
-  if (rc) return rc;
-  db = static_cast<BrushDev*>(p);
-  if (n > 0) CK(cudaMemcpyAsync(db, brushes, sizeof(BrushDev) * n, cudaMemcpyHostToDevice, s));
+  int n = std::min(count, kMaxBrushes);  // builder.ts:57,148-153
+  // the volume keeps its brush buffer (an allocation and a free per build cost more than the fold)
+  if (!v->brushes) {
+    void* p = nullptr;
+    int rc = v->ctx->dev_alloc(&p, sizeof(BrushDev) * kMaxBrushes);
+    if (rc) return rc;
+    v->brushes = static_cast<BrushDev*>(p);
+  }
+  if (n > 0) CK(cudaMemcpyAsync(v->brushes, brushes, sizeof(BrushDev) * n, cudaMemcpyHostToDevice, s));
+  BuildDev B;
+  B.levels = v->mips;
+  int64_t tiles = 0;
   for (int m = 0; m < v->mips; m++) {
     double voxel = (v->world / v->res) * std::pow(2.0, m);
     double tile_size = voxel * TILE;
     double bw = v->band * voxel;
-    BuildLevelDev L;
+    BuildLevelDev& L = B.level[m];
     L.dist = v->dist + v->off[m];
     L.mat = v->mat + v->off[m];
     L.R = v->res >> m;
     L.tiles = v->tile_res[m];
+    tiles += static_cast<int64_t>(L.tiles) * L.tiles * L.tiles;
     // The builder bakes the origin the volume had at construction (builder.ts:75).
     L.ox = static_cast<float>(v->origin[0]);
     L.oy = static_cast<float>(v->origin[1]);
@@ -774,10 +783,9 @@ int clay_volume_build_brushes(clay_volume* v, const clay_brush* brushes, int cou
     L.tile_half = static_cast<float>(tile_size / 2);
     L.bw = static_cast<float>(bw);
     L.empty = static_cast<float>(bw * 4);
-    CK(L_build(L, db, n, s));
   }
+  CK(L_build(B, static_cast<int>(tiles), v->brushes, n, s));
   CK(cudaStreamSynchronize(s));
-  v->ctx->dev_free(db, sizeof(BrushDev) * std::max(n, 1));
   return CLAY_OK;
 }
 

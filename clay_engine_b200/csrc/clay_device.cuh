@@ -295,6 +295,11 @@ struct BuildLevelDev {
   int32_t R, tiles;
   float ox, oy, oz, voxel, tile_size, tile_half, bw, empty;
 };
+struct BuildDev {
+  BuildLevelDev level[kMaxMips];
+  int32_t levels;
+};
+constexpr uint32_t kBuildKeep = 64;  // brushes a tile folds (builder.ts:57)
 
 }  // namespace clay
 
@@ -2846,8 +2851,19 @@ __device__ __forceinline__ float smoothstepf(float e0, float e1, float x) {
   return t * t * (3.0f - 2.0f * t);
 }
 
-__device__ __forceinline__ void apply_brush(float& ax, float& ay, const BrushDev& b, float px, float py, float pz) {
-  float inv_scale = __frcp_rn(fmaxf(b.scale, 1e-5f));
+// clamp(0.5 + num / k, 0, 1) for k > 0, without the division where the quotient is at least a half away from
+// zero: the rounded quotient is then at or beyond the half too, and the clamp gives exactly 0 or 1.
+__device__ __forceinline__ float blend_weight(float num, float k) {
+  const float half = 0.5f * k;
+  if (half < __int_as_float(0x7f800000)) {  // inf / inf is not a number
+    if (num >= half) return 1.0f;
+    if (num <= -half) return 0.0f;
+  }
+  return clampf(0.5f + __fdiv_rn(num, k), 0.0f, 1.0f);
+}
+
+// inv_scale: 1 / max(b.scale, 1e-5)
+__device__ __forceinline__ void apply_brush(float& ax, float& ay, const BrushDev& b, float inv_scale, float px, float py, float pz) {
   float qx = -b.rot[0], qy = -b.rot[1], qz = -b.rot[2], qw = b.rot[3];
   float vx = px - b.pos[0], vy = py - b.pos[1], vz = pz - b.pos[2];
   float tx = (qy * vz - qz * vy) * 2.0f, ty = (qz * vx - qx * vz) * 2.0f, tz = (qx * vy - qy * vx) * 2.0f;
@@ -2858,7 +2874,7 @@ __device__ __forceinline__ void apply_brush(float& ax, float& ay, const BrushDev
   float keep = b.mask >= 0.0f ? 1.0f - smoothstepf(0.25f, 0.75f, fabsf(ay - b.mask)) : 1.0f;
   if (b.op == 0u) {
     float kk = fmaxf(b.blend, 1e-6f);
-    float h = clampf(0.5f + __fdiv_rn(0.5f * (ax - dist), kk), 0.0f, 1.0f);
+    float h = blend_weight(0.5f * (ax - dist), kk);
     float rx = (ax * (1.0f - h) + dist * h) - kk * h * (1.0f - h);
     float ny = ay * (1.0f - h) + b.material * h;
     float nax = ax * (1.0f - keep) + rx * keep;
@@ -2868,7 +2884,7 @@ __device__ __forceinline__ void apply_brush(float& ax, float& ay, const BrushDev
   } else if (b.op == 1u) {
     float a = -dist;
     float kk = fmaxf(b.blend, 1e-6f);
-    float h = clampf(0.5f - __fdiv_rn(0.5f * (ax - a), kk), 0.0f, 1.0f);
+    float h = blend_weight(-(0.5f * (ax - a)), kk);
     float rx = (ax * (1.0f - h) + a * h) + kk * h * (1.0f - h);
     float hh = h * 0.85f;
     float ny = ay * (1.0f - hh) + b.material * hh;
@@ -2883,27 +2899,53 @@ __device__ __forceinline__ void apply_brush(float& ax, float& ay, const BrushDev
   }
 }
 
-__global__ void __launch_bounds__(256) k_build(const BuildLevelDev L, const BrushDev* __restrict__ brushes, int nbrush) {
-  __shared__ int s_ids[64];
-  __shared__ int s_n;
-  const int wx = blockIdx.x, wy = blockIdx.y, wz = blockIdx.z;
+// A block per 8^3 tile, all levels in one launch, the coarsest first (their tiles meet the most
+// brushes). The cull tests a brush per thread (one thread testing 64 brushes one after another was most
+// of a coarse level: 51-76 us each, at any size), keeps the first 64 in order, and the kept records
+// are folded from shared memory. Bound by the fold's FP32 work: 192^3 x 4 levels from 64 brushes, a call with
+// its upload and wait: 323 us before, 100 now.
+__global__ void __launch_bounds__(256) k_build(const BuildDev B, const BrushDev* __restrict__ brushes, int nbrush) {
+  __shared__ BrushDev s_brush[kBuildKeep];
+  __shared__ float s_inv[kBuildKeep];
+  __shared__ uint32_t s_warp[8];
+  uint32_t t = blockIdx.x;
+  int m = B.levels - 1;
+  for (; m > 0; m--) {
+    const uint32_t n = static_cast<uint32_t>(B.level[m].tiles) * B.level[m].tiles * B.level[m].tiles;
+    if (t < n) break;
+    t -= n;
+  }
+  const BuildLevelDev& L = B.level[m];
+  const uint32_t tiles = static_cast<uint32_t>(L.tiles);
+  const int wx = static_cast<int>(t % tiles), wy = static_cast<int>((t / tiles) % tiles), wz = static_cast<int>(t / (tiles * tiles));
   const float tminx = L.ox + static_cast<float>(wx) * L.tile_size;
   const float tminy = L.oy + static_cast<float>(wy) * L.tile_size;
   const float tminz = L.oz + static_cast<float>(wz) * L.tile_size;
-  if (threadIdx.x == 0) {
-    float tcx = tminx + L.tile_half, tcy = tminy + L.tile_half, tcz = tminz + L.tile_half;
-    int n = 0;
-    for (int b = 0; b < nbrush; b++) {
-      const BrushDev& B = brushes[b];
-      float nx = fmaxf(fabsf(B.pos[0] - tcx) - L.tile_half, 0.0f);
-      float ny = fmaxf(fabsf(B.pos[1] - tcy) - L.tile_half, 0.0f);
-      float nz = fmaxf(fabsf(B.pos[2] - tcz) - L.tile_half, 0.0f);
-      if (len3(nx, ny, nz) < B.bound + L.bw && n < 64) s_ids[n++] = b;
-    }
-    s_n = n;
+  const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+  bool keep = false;
+  if (static_cast<int>(threadIdx.x) < nbrush) {  // at most 256
+    const BrushDev& q = brushes[threadIdx.x];
+    const float tcx = tminx + L.tile_half, tcy = tminy + L.tile_half, tcz = tminz + L.tile_half;
+    const float nx = fmaxf(fabsf(q.pos[0] - tcx) - L.tile_half, 0.0f);
+    const float ny = fmaxf(fabsf(q.pos[1] - tcy) - L.tile_half, 0.0f);
+    const float nz = fmaxf(fabsf(q.pos[2] - tcz) - L.tile_half, 0.0f);
+    keep = len3(nx, ny, nz) < q.bound + L.bw;
+  }
+  const uint32_t kept = __ballot_sync(0xffffffffu, keep);
+  if (lane == 0) s_warp[wid] = __popc(kept);
+  __syncthreads();
+  uint32_t before = 0, all = 0;
+  for (uint32_t k = 0; k < 8; k++) {
+    if (k < wid) before += s_warp[k];
+    all += s_warp[k];
+  }
+  const uint32_t place = before + __popc(kept & ((1u << lane) - 1u));
+  if (keep && place < kBuildKeep) {
+    s_brush[place] = brushes[threadIdx.x];
+    s_inv[place] = __frcp_rn(fmaxf(s_brush[place].scale, 1e-5f));
   }
   __syncthreads();
-  const int n = s_n;
+  const uint32_t n = min(all, kBuildKeep);
   const int lx = threadIdx.x & 7, ly = (threadIdx.x >> 3) & 7, lz2 = threadIdx.x >> 6;
   for (int half = 0; half < 2; half++) {
     int lz = lz2 * 2 + half;
@@ -2911,7 +2953,7 @@ __global__ void __launch_bounds__(256) k_build(const BuildLevelDev L, const Brus
     float py = tminy + (static_cast<float>(ly) + 0.5f) * L.voxel;
     float pz = tminz + (static_cast<float>(lz) + 0.5f) * L.voxel;
     float ax = L.empty, ay = 0.0f;
-    for (int q = 0; q < n; q++) apply_brush(ax, ay, brushes[s_ids[q]], px, py, pz);
+    for (uint32_t q = 0; q < n; q++) apply_brush(ax, ay, s_brush[q], s_inv[q], px, py, pz);
     int x = wx * 8 + lx, y = wy * 8 + ly, z = wz * 8 + lz;
     size_t idx = static_cast<size_t>(x) + static_cast<size_t>(L.R) * (static_cast<size_t>(y) + static_cast<size_t>(L.R) * z);
     L.dist[idx] = __float2half_rn(clampf(__fdiv_rn(ax, L.bw), -1.0f, 1.0f));

@@ -127,9 +127,8 @@ cudaError_t L_ext_qemit(const ExtractDev* e, int blocks, cudaStream_t st) {
   CLAY_LAUNCH(k_ext_qemit, blocks, kExtractThreads, st, e);
 }
 cudaError_t L_ext_finish(const ExtractDev* e, cudaStream_t st) { CLAY_LAUNCH(k_ext_finish, 1, kExtractThreads, st, e); }
-cudaError_t L_build(const BuildLevelDev& lv, const BrushDev* brushes, int n, cudaStream_t st) {
-  dim3 g(lv.tiles, lv.tiles, lv.tiles);
-  CLAY_LAUNCH(k_build, g, 256, st, lv, brushes, n);
+cudaError_t L_build(const BuildDev& b, int tiles, const BrushDev* brushes, int n, cudaStream_t st) {
+  CLAY_LAUNCH(k_build, tiles, 256, st, b, brushes, n);
 }
 cudaError_t L_cell_index(const SceneDev* s, uint32_t* out, int n, cudaStream_t st) {
   CLAY_LAUNCH(k_cell_index, (n + 255) / 256, 256, st, s, out);

@@ -123,3 +123,16 @@ def test_rgba16f_export_has_the_reference_texel_layout(root, oracle):
     assert (t[..., 0] == lvl).all()
     assert (t[..., 2] == 0).all() and (t[..., 3] == 0x3C00).all()
     v.destroy()
+
+
+@pytest.mark.parametrize("n, res", [(0, 16), (1, 8), (33, 40), (64, 32), (90, 64), (256, 16), (300, 16)])
+def test_build_brush_counts_are_bit_exact(root, oracle, n, res):
+    """The cull takes a brush per thread and keeps a tile's first 64 in order: no brush, one, over a
+    warp, the tile's limit and beyond it (large overlapping brushes), the list's limit and beyond it."""
+    from clay_engine_b200 import scenes
+
+    b = scenes.random_brushes(n, seed=n, radius=(3.0, 9.0)) if n else np.zeros(0, scenes.config1_collider_brushes().dtype)
+    v, gd, gm, od, om = build_both(root, oracle, b, res)
+    assert (gd == od).all(), f"{(gd != od).sum()} distance texels differ"
+    assert (gm == om).all()
+    v.destroy()
