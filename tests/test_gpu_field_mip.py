@@ -87,3 +87,27 @@ def test_device_points_match_the_host_hook(root, oracle):
         f.query_mip_device(dp.cpu(), s, g, 0)
     f.destroy()
     v.destroy()
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+def test_rows_of_texels_end_to_end(root, shift):
+    """Points at every place of a row's groups of four texels, both edges included, into outputs that are 8-byte
+    aligned or only 4: the device query equals the host one at the same points."""
+    import torch
+
+    import clay_engine_b200 as ce
+    from clay_engine_b200 import scenes
+
+    vol = ce.SdfVolume(root, resolution=16, worldSize=16.0, origin=(0.0, 0.0, 0.0), mipLevels=2)
+    vol.build(scenes.random_brushes(6, seed=3, lo=(2, 2, 2), hi=(14, 14, 14)))
+    field = ce.volumeField(vol)
+    x = np.linspace(-0.25, 16.25, 133, dtype=np.float32)
+    pts = np.stack([x, np.roll(x, 17).clip(0, 16), np.roll(x, 71).clip(0, 16)], 1)
+    dp = torch.from_numpy(pts).cuda()
+    for mip in (0, 1):
+        out = [torch.zeros(2 * len(pts) + 1, device="cuda")[shift:shift + 2 * len(pts)].view(-1, 2) for _ in range(2)]
+        field.query_mip_device(dp, out[0], out[1], mip)
+        torch.cuda.synchronize()
+        s, f = field.query_mip(pts, mip)
+        assert np.array_equal(out[0].cpu().numpy(), s) and np.array_equal(out[1].cpu().numpy(), f)
+        assert len(np.unique(s[:, 1])) > 20
