@@ -2329,7 +2329,7 @@ struct clay_extractor {
   std::vector<DevBuf> bufs;
   bool dirty = true;
   int blocks = 0;
-  // the eight passes of one extraction, captured on the first extract and replayed after:
+  // the passes of one extraction, captured on the first extract and replayed after:
   // every pass reads its parameters from `d`, so one graph serves every region and motion
   cudaGraphExec_t graph = nullptr;
   int64_t launches = 0;
@@ -2438,21 +2438,22 @@ int clay_extractor_extract(clay_extractor* x, void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   int rc = x->flush(s);
   if (rc) return rc;
-  // A small lattice (the game's 32^3 per body) is bound by launching its eight dependent
+  // A small lattice (the game's 32^3 per body) is bound by launching its four dependent
   // passes, so they run as one CUDA graph, captured on a private stream at the first call.
   if (!x->graph) {
     cudaStream_t cs;
     CK(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
     CK(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
     const uint64_t before = launch_count();
-    cudaError_t e = L_ext_reset(x->d, cs);
+    const bool scans = x->blocks > kExtractInline;
+    cudaError_t e = cudaSuccess;
+    if (x->h.has_motion) e = L_ext_reset(x->d, cs);
     if (e == cudaSuccess) e = L_ext_cells(x->d, x->blocks, cs);
-    if (e == cudaSuccess) e = L_ext_scan(x->d, 0, cs);
+    if (e == cudaSuccess && scans) e = L_ext_scan(x->d, 0, cs);
     if (e == cudaSuccess) e = L_ext_emit(x->d, x->blocks, cs);
     if (e == cudaSuccess) e = L_ext_qcount(x->d, x->blocks, cs);
-    if (e == cudaSuccess) e = L_ext_scan(x->d, 1, cs);
+    if (e == cudaSuccess && scans) e = L_ext_scan(x->d, 1, cs);
     if (e == cudaSuccess) e = L_ext_qemit(x->d, x->blocks, cs);
-    if (e == cudaSuccess) e = L_ext_finish(x->d, cs);
     x->launches = static_cast<int64_t>(launch_count() - before);
     cudaGraph_t g = nullptr;
     const cudaError_t ec = cudaStreamEndCapture(cs, &g);

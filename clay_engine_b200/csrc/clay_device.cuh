@@ -240,10 +240,12 @@ struct __align__(16) ExtractDev {
   unsigned char* bodies;
   float* motion;
   uint32_t* id_grid;   // res^3, +1 biased particle index, 0: no dual vertex
-  float4* rec;         // res^3 x 2: (vertex, material), (normal, has-vertex)
+  float4* rec;         // res^3 x 2: (vertex, material), (normal, -) where id_grid holds a vertex mark
   uint32_t* blk;       // per block of 256 cells: vertex count, then its exclusive offset
   uint32_t* qblk;      // per block of 256 lattice points: quad count, then offset
-  unsigned char* qmask;  // res^3: the edges (x, y, z bits) whose quad is emitted
+  // res^3: bits 0-2 the edges (+x, +y, +z) that straddle the surface, after the count pass those whose
+  // quad is emitted; bit 3: the low end lies outside
+  unsigned char* qmask;
   uint32_t* indices;   // quad_cap x 6
   uint32_t* draw_args; // vertexCount, instanceCount, firstVertex, firstInstance
   uint32_t* counters;  // vertex cells, quads (before the capacity clamps)
@@ -254,6 +256,7 @@ struct __align__(16) ExtractDev {
   int32_t res, body, base, capacity, quad_cap, has_motion, nblocks, pad_;
 };
 constexpr int kExtractThreads = 256;  // cells (lattice points) per block of the grid passes
+constexpr int kExtractInline = 1024;  // blocks up to which they add up the counts before them
 
 // A ClaySolver (sim/pbd.ts:78-424) as the kernels see it: the caller's ParticleSet records,
 // the world field and the SolveParams uniform (pbd.ts:12-41).
@@ -3109,6 +3112,26 @@ __device__ __forceinline__ uint32_t ext_block_scan(uint32_t v, uint32_t& excl) {
   return total;
 }
 
+// What the blocks before this one counted (`which` 0: vertices, 1: quads). Up to kExtractInline blocks every
+// block adds up the counts before it, which costs less than a scan launched between two passes; above, k_ext_scan
+// has turned the counts into their prefix. The last block also leaves the total.
+__device__ __forceinline__ uint32_t ext_before(const ExtractDev& E, int which, uint32_t block) {
+  const uint32_t* a = which == 0 ? E.blk : E.qblk;
+  if (E.nblocks > kExtractInline) return a[block];
+  __shared__ uint32_t s_part[kExtractThreads / 32];
+  const uint32_t last = static_cast<uint32_t>(E.nblocks) - 1u, lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+  uint32_t v = 0;
+  for (uint32_t i = threadIdx.x; i < block; i += kExtractThreads) v += a[i];
+  v = __reduce_add_sync(0xffffffffu, v);
+  if (lane == 0) s_part[wid] = v;
+  __syncthreads();
+  uint32_t sum = 0;
+  for (uint32_t k = 0; k < kExtractThreads / 32; k++) sum += s_part[k];
+  __syncthreads();
+  if (block == last && threadIdx.x == 0) E.counters[which] = sum + a[last];
+  return sum;
+}
+
 // The scan origin (extract.ts:169-178) and the emitted velocity (:179-188).
 __device__ __forceinline__ void ext_origin(const ExtractDev& E, float& ox, float& oy, float& oz) {
   ox = E.origin[0];
@@ -3127,16 +3150,62 @@ __device__ __forceinline__ float ext_dist(const ExtractDev& E, float px, float p
   return sx;
 }
 
-// reset (extract.ts:194-246): with motion and preserveMotion, the centre and mean velocity of
+// The field's distances at a cell's eight corners (x0 or x1, y0 or y1, z0 or z1; corner i takes bit 0, 1, 2 of i),
+// the same operations as ext_dist at each: what depends on one axis alone (the offset, the box test's term, the
+// division by the extent, the texel indices and the fraction) is done once per axis and end instead of at
+// every corner.
+__device__ __forceinline__ void ext_corners(const ExtractDev& E, const float (&px)[2], const float (&py)[2], const float (&pz)[2],
+                                            float (&d)[8]) {
+  const FieldDev* f = E.field;
+#pragma unroll
+  for (int i = 0; i < 8; i++) d[i] = 0.0f;
+  for (int k = 0; k < f->n; k++) {
+    const LeafDev& lf = f->leaf[k];
+    const Vol v = load_vol(lf.vp);
+    const float bw = v.band * v.voxel * 1.0f;
+    float c[3][2], fr[3][2];  // per axis and end: the box test's term, the fraction
+    int i0[3][2], i1[3][2];
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      float q[3];
+      leaf_point(lf, px[e], py[e], pz[e], q[0], q[1], q[2]);  // each axis by itself
+      const float o[3] = {v.ox, v.oy, v.oz}, m[3] = {v.cx, v.cy, v.cz};
+#pragma unroll
+      for (int a = 0; a < 3; a++) {
+        c[a][e] = fabsf(q[a] - m[a]) - v.half;
+        tri_axis(__fdiv_rn(q[a] - o[a], v.extent), v.res, i0[a][e], i1[a][e], fr[a][e]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const int ex = i & 1, ey = (i >> 1) & 1, ez = i >> 2;
+      const float qx = c[0][ex], qy = c[1][ey], qz = c[2][ez];
+      float s;
+      float dbox = -1.0f;  // inside, unless a term says otherwise (the terms' maximum is then negative or zero)
+      if (!(qx <= 0.0f && qy <= 0.0f && qz <= 0.0f)) {
+        const float mx = fmaxf(qx, 0.0f), my = fmaxf(qy, 0.0f), mz = fmaxf(qz, 0.0f);
+        dbox = len3(mx, my, mz) + fminf(fmaxf(qx, fmaxf(qy, qz)), 0.0f);
+      }
+      if (dbox > 0.0f) {
+        s = dbox;
+      } else {
+        auto at = [&](int y, int z) {
+          return lerpf(texel(v, i0[0][ex], y, z), texel(v, i1[0][ex], y, z), fr[0][ex]);
+        };
+        const float c0 = lerpf(at(i0[1][ey], i0[2][ez]), at(i1[1][ey], i0[2][ez]), fr[1][ey]);
+        const float c1 = lerpf(at(i0[1][ey], i1[2][ez]), at(i1[1][ey], i1[2][ez]), fr[1][ey]);
+        s = lerpf(c0, c1, fr[2][ez]) * bw;
+      }
+      if (k == 0 || !(d[i] < s)) d[i] = s;
+    }
+  }
+}
+
+// reset (extract.ts:194-246), launched for an extractor with motion: with preserveMotion, the centre and mean velocity of
 // the body's current particles (per-thread strided sums, then a tree) become the motion.
 __global__ void __launch_bounds__(kExtractThreads) k_ext_reset(const ExtractDev* __restrict__ e) {
   const ExtractDev& E = *e;
   const uint32_t li = threadIdx.x;
-  if (li == 0) {
-    E.counters[0] = 0u;
-    E.counters[1] = 0u;
-  }
-  if (!E.has_motion) return;
   __shared__ float s_sum[kExtractThreads][6];
   const unsigned char* bd = E.bodies + static_cast<size_t>(E.body) * 64;
   const uint32_t first = *reinterpret_cast<const uint32_t*>(bd + 12);
@@ -3203,10 +3272,22 @@ __global__ void __launch_bounds__(kExtractThreads) k_ext_cells(const ExtractDev*
     const float c = E.cell;
     const float x0 = ox + static_cast<float>(gx) * c, y0 = oy + static_cast<float>(gy) * c, z0 = oz + static_cast<float>(gz) * c;
     const float x1 = x0 + c, y1 = y0 + c, z1 = z0 + c;
-    const float d0 = ext_dist(E, x0, y0, z0), dx = ext_dist(E, x1, y0, z0), dy = ext_dist(E, x0, y1, z0),
-                dz = ext_dist(E, x0, y0, z1), dxy = ext_dist(E, x1, y1, z0), dxz = ext_dist(E, x1, y0, z1),
-                dyz = ext_dist(E, x0, y1, z1), dxyz = ext_dist(E, x1, y1, z1);
+    float d[8];
+    ext_corners(E, {x0, x1}, {y0, y1}, {z0, z1}, d);
+    const float d0 = d[0], dx = d[1], dy = d[2], dxy = d[3], dz = d[4], dxz = d[5], dyz = d[6], dxyz = d[7];
+    // a quad's edges straddle by the same samples as the cell's (extract.ts:352-392)
+    E.qmask[idx] = static_cast<unsigned char>((dx * d0 < 0.0f ? 1u : 0u) | (dy * d0 < 0.0f ? 2u : 0u) | (dz * d0 < 0.0f ? 4u : 0u) |
+                                              (d0 < 0.0f ? 0u : 8u));
+    float low = d0, high = d0, sum = d0;
+#pragma unroll
+    for (int i = 1; i < 8; i++) {
+      low = fminf(low, d[i]);
+      high = fmaxf(high, d[i]);
+      sum += d[i];
+    }
     float ax = 0.0f, ay = 0.0f, az = 0.0f, aw = 0.0f;
+    // no edge crosses where no two corners differ in sign (a sum that is not a number: see for each)
+    if (!(low >= 0.0f) && !(high <= 0.0f) || sum != sum) {
     // the twelve edges in the reference's order
     ext_cross(x0, y0, z0, d0, x1, y0, z0, dx, ax, ay, az, aw);
     ext_cross(x0, y1, z0, dy, x1, y1, z0, dxy, ax, ay, az, aw);
@@ -3220,7 +3301,7 @@ __global__ void __launch_bounds__(kExtractThreads) k_ext_cells(const ExtractDev*
     ext_cross(x1, y0, z0, dx, x1, y0, z1, dxz, ax, ay, az, aw);
     ext_cross(x0, y1, z0, dy, x0, y1, z1, dyz, ax, ay, az, aw);
     ext_cross(x1, y1, z0, dxy, x1, y1, z1, dxyz, ax, ay, az, aw);
-    float4 r0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), r1 = r0;
+    }
     if (!(aw < 0.5f)) {
       const float inv = __fdiv_rn(1.0f, aw);
       const float vx = ax * inv, vy = ay * inv, vz = az * inv;
@@ -3237,12 +3318,11 @@ __global__ void __launch_bounds__(kExtractThreads) k_ext_cells(const ExtractDev*
         const int ch = field_pick(E.field, px, py, pz, s0, s1);
         mat = field_material(E.field, ch, px, py, pz);
       }
-      r0 = make_float4(px, py, pz, mat);
-      r1 = make_float4(nx, ny, nz, 1.0f);
+      E.rec[2 * static_cast<size_t>(idx)] = make_float4(px, py, pz, mat);
+      E.rec[2 * static_cast<size_t>(idx) + 1] = make_float4(nx, ny, nz, 0.0f);
       has = 1;
     }
-    E.rec[2 * static_cast<size_t>(idx)] = r0;
-    E.rec[2 * static_cast<size_t>(idx) + 1] = r1;
+    E.id_grid[idx] = has;
   }
   uint32_t excl;
   const uint32_t total = ext_block_scan(has, excl);
@@ -3297,20 +3377,17 @@ __global__ void __launch_bounds__(kExtractThreads) k_ext_emit(const ExtractDev* 
   const uint32_t R = static_cast<uint32_t>(E.res);
   const uint32_t idx = blockIdx.x * kExtractThreads + threadIdx.x;
   const bool in = idx < R * R * R;
-  float4 r0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), r1 = r0;
-  if (in) {
-    r0 = E.rec[2 * static_cast<size_t>(idx)];
-    r1 = E.rec[2 * static_cast<size_t>(idx) + 1];
-  }
-  const uint32_t has = (in && r1.w > 0.5f) ? 1u : 0u;
+  const uint32_t has = in ? E.id_grid[idx] : 0u;
+  const uint32_t before = ext_before(E, 0, blockIdx.x);
   uint32_t excl;
   ext_block_scan(has, excl);
-  if (!in) return;
-  const uint32_t slot = E.blk[blockIdx.x] + excl;
-  if (!has || slot >= static_cast<uint32_t>(E.capacity)) {
+  if (!has) return;
+  const uint32_t slot = before + excl;
+  if (slot >= static_cast<uint32_t>(E.capacity)) {
     E.id_grid[idx] = 0u;
     return;
   }
+  const float4 r0 = E.rec[2 * static_cast<size_t>(idx)], r1 = E.rec[2 * static_cast<size_t>(idx) + 1];
   const uint32_t id = static_cast<uint32_t>(E.base) + slot;
   float vx = E.vel[0], vy = E.vel[1], vz = E.vel[2];
   if (E.has_motion) {
@@ -3334,29 +3411,24 @@ __device__ __forceinline__ uint32_t ext_id(const ExtractDev& E, uint32_t x, uint
 }
 
 // The three quads a lattice point may own (extract.ts:352-392): for edge a (0: +x, 1: +y,
-// 2: +z) whose ends straddle the surface, the ids of the four cells around it in the
+// 2: +z), whose ends straddle the surface, the ids of the four cells around it in the
 // reference's order; all four must hold a vertex.
-__device__ __forceinline__ bool ext_quad(const ExtractDev& E, uint32_t i, uint32_t j, uint32_t k, int a, float dL, float lx,
-                                         float ly, float lz, uint32_t q[4]) {
+__device__ __forceinline__ bool ext_quad(const ExtractDev& E, uint32_t i, uint32_t j, uint32_t k, int a, uint32_t q[4]) {
   const uint32_t hi = static_cast<uint32_t>(E.res) - 1u;
-  const float c = E.cell;
   if (a == 0) {
     if (!(j >= 1 && k >= 1 && j <= hi && k <= hi)) return false;
-    if (!(ext_dist(E, lx + c, ly + 0.0f, lz + 0.0f) * dL < 0.0f)) return false;
     q[0] = ext_id(E, i, j - 1, k - 1);
     q[1] = ext_id(E, i, j, k - 1);
     q[2] = ext_id(E, i, j, k);
     q[3] = ext_id(E, i, j - 1, k);
   } else if (a == 1) {
     if (!(i >= 1 && k >= 1 && i <= hi && k <= hi)) return false;
-    if (!(ext_dist(E, lx + 0.0f, ly + c, lz + 0.0f) * dL < 0.0f)) return false;
     q[0] = ext_id(E, i - 1, j, k - 1);
     q[1] = ext_id(E, i - 1, j, k);
     q[2] = ext_id(E, i, j, k);
     q[3] = ext_id(E, i, j, k - 1);
   } else {
     if (!(i >= 1 && j >= 1 && i <= hi && j <= hi)) return false;
-    if (!(ext_dist(E, lx + 0.0f, ly + 0.0f, lz + c) * dL < 0.0f)) return false;
     q[0] = ext_id(E, i - 1, j - 1, k);
     q[1] = ext_id(E, i, j - 1, k);
     q[2] = ext_id(E, i, j, k);
@@ -3365,60 +3437,59 @@ __device__ __forceinline__ bool ext_quad(const ExtractDev& E, uint32_t i, uint32
   return q[0] != 0u && q[1] != 0u && q[2] != 0u && q[3] != 0u;
 }
 
-// quads, pass 1: which of a lattice point's edges emit, and the block's count.
+// quads, pass 1: which of a lattice point's straddling edges emit, and the block's count.
 __global__ void __launch_bounds__(kExtractThreads) k_ext_qcount(const ExtractDev* __restrict__ e) {
   const ExtractDev& E = *e;
   const uint32_t R = static_cast<uint32_t>(E.res);
   const uint32_t idx = blockIdx.x * kExtractThreads + threadIdx.x;
   uint32_t m = 0;
   if (idx < R * R * R) {
-    const uint32_t i = idx % R, j = (idx / R) % R, k = idx / (R * R);
-    float ox, oy, oz;
-    ext_origin(E, ox, oy, oz);
-    const float c = E.cell;
-    const float lx = ox + static_cast<float>(i) * c, ly = oy + static_cast<float>(j) * c, lz = oz + static_cast<float>(k) * c;
-    const float dL = ext_dist(E, lx, ly, lz);
-    uint32_t q[4];
-    for (int a = 0; a < 3; a++)
-      if (ext_quad(E, i, j, k, a, dL, lx, ly, lz, q)) m |= 1u << a;
-    E.qmask[idx] = static_cast<unsigned char>(m);
+    const uint32_t edges = E.qmask[idx];
+    if (edges & 7u) {
+      const uint32_t i = idx % R, j = (idx / R) % R, k = idx / (R * R);
+      uint32_t q[4];
+      for (int a = 0; a < 3; a++)
+        if (((edges >> a) & 1u) && ext_quad(E, i, j, k, a, q)) m |= 1u << a;
+      if (m != (edges & 7u)) E.qmask[idx] = static_cast<unsigned char>((edges & 8u) | m);
+    }
   }
   uint32_t excl;
   const uint32_t total = ext_block_scan(static_cast<uint32_t>(__popc(m)), excl);
   if (threadIdx.x == 0) E.qblk[blockIdx.x] = total;
 }
 
-// quads, pass 2: six indices per quad (extract.ts:330-350), wound by the sign at the low end.
+__device__ __forceinline__ void ext_finish(const ExtractDev& E);
+
+// quads, pass 2: six indices per quad (extract.ts:330-350), wound by the sign at the low end. The first
+// block finishes the extraction beside the others (a launch of its own took 24 us for 39,000 particles).
 __global__ void __launch_bounds__(kExtractThreads) k_ext_qemit(const ExtractDev* __restrict__ e) {
   const ExtractDev& E = *e;
+  if (blockIdx.x == 0) {
+    ext_finish(E);
+    return;
+  }
+  const uint32_t block = blockIdx.x - 1u;
   const uint32_t R = static_cast<uint32_t>(E.res);
-  const uint32_t idx = blockIdx.x * kExtractThreads + threadIdx.x;
+  const uint32_t idx = block * kExtractThreads + threadIdx.x;
   const bool in = idx < R * R * R;
-  const uint32_t m = in ? static_cast<uint32_t>(E.qmask[idx]) : 0u;
+  const uint32_t edges = in ? static_cast<uint32_t>(E.qmask[idx]) : 0u, m = edges & 7u;
+  const uint32_t before = ext_before(E, 1, block);
   uint32_t excl;
   ext_block_scan(static_cast<uint32_t>(__popc(m)), excl);
   if (!m) return;
   const uint32_t i = idx % R, j = (idx / R) % R, k = idx / (R * R);
-  float ox, oy, oz;
-  ext_origin(E, ox, oy, oz);
-  const float c = E.cell;
-  const float lx = ox + static_cast<float>(i) * c, ly = oy + static_cast<float>(j) * c, lz = oz + static_cast<float>(k) * c;
-  const float dL = ext_dist(E, lx, ly, lz);
-  const bool flip = !(dL < 0.0f);
-  uint32_t slot = E.qblk[blockIdx.x] + excl;
+  const bool flip = (edges & 8u) != 0u;
+  uint32_t slot = before + excl;
   for (int a = 0; a < 3; a++) {
     if (!(m & (1u << a))) continue;
     uint32_t q[4];
-    ext_quad(E, i, j, k, a, dL, lx, ly, lz, q);
+    ext_quad(E, i, j, k, a, q);
     if (slot < static_cast<uint32_t>(E.quad_cap)) {
-      uint32_t* o = E.indices + static_cast<size_t>(slot) * 6;
+      uint2* o = reinterpret_cast<uint2*>(E.indices + static_cast<size_t>(slot) * 6);
       const uint32_t i0 = q[0] - 1u, i1 = (flip ? q[3] : q[1]) - 1u, i2 = q[2] - 1u, i3 = (flip ? q[1] : q[3]) - 1u;
-      o[0] = i0;
-      o[1] = i1;
-      o[2] = i2;
-      o[3] = i0;
-      o[4] = i2;
-      o[5] = i3;
+      o[0] = make_uint2(i0, i1);
+      o[1] = make_uint2(i2, i0);
+      o[2] = make_uint2(i2, i3);
     }
     slot++;
   }
@@ -3426,17 +3497,35 @@ __global__ void __launch_bounds__(kExtractThreads) k_ext_qemit(const ExtractDev*
 
 // finish (extract.ts:395-436): the body record (first, count, rest centre of mass, rotation
 // reset) and the draw arguments.
-__global__ void __launch_bounds__(kExtractThreads) k_ext_finish(const ExtractDev* __restrict__ e) {
-  const ExtractDev& E = *e;
+__device__ __forceinline__ void ext_finish(const ExtractDev& E) {
   const uint32_t li = threadIdx.x;
   const uint32_t n = min(E.counters[0], static_cast<uint32_t>(E.capacity));
   __shared__ float s_g[kExtractThreads][3];
+  __shared__ uint32_t s_quads;
+  // the quads in all: the scan's total, or (added up by the blocks themselves) every block's count
+  if (li == 0) s_quads = E.nblocks > kExtractInline ? E.counters[1] : 0u;
+  __syncthreads();
+  if (E.nblocks <= kExtractInline) {
+    uint32_t v = 0;
+    for (uint32_t i = li; i < static_cast<uint32_t>(E.nblocks); i += kExtractThreads) v += E.qblk[i];
+    v = __reduce_add_sync(0xffffffffu, v);
+    if ((li & 31u) == 0) atomicAdd(&s_quads, v);
+  }
+  // a thread's particles in order, eight loaded before any is added (this block alone waits on them)
   float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-  for (uint32_t t = li; t < n; t += kExtractThreads) {
-    const float* p = reinterpret_cast<const float*>(E.particles + static_cast<size_t>(E.base + t) * 96 + 64);  // rest
-    sx = sx + p[0];
-    sy = sy + p[1];
-    sz = sz + p[2];
+  for (uint32_t t = li; t < n; t += 8 * kExtractThreads) {
+    float4 p[8];
+#pragma unroll
+    for (uint32_t u = 0; u < 8; u++)
+      if (t + u * kExtractThreads < n)
+        p[u] = *reinterpret_cast<const float4*>(E.particles + static_cast<size_t>(E.base + t + u * kExtractThreads) * 96 + 64);  // rest
+#pragma unroll
+    for (uint32_t u = 0; u < 8; u++)
+      if (t + u * kExtractThreads < n) {
+        sx = sx + p[u].x;
+        sy = sy + p[u].y;
+        sz = sz + p[u].z;
+      }
   }
   s_g[li][0] = sx;
   s_g[li][1] = sy;
@@ -3465,7 +3554,7 @@ __global__ void __launch_bounds__(kExtractThreads) k_ext_finish(const ExtractDev
   f[5] = 0.0f;
   f[6] = 0.0f;
   f[7] = 1.0f;
-  const uint32_t q = min(E.counters[1], static_cast<uint32_t>(E.quad_cap));
+  const uint32_t q = min(s_quads, static_cast<uint32_t>(E.quad_cap));
   E.draw_args[0] = q * 6u;
   E.draw_args[1] = 1u;
   E.draw_args[2] = 0u;

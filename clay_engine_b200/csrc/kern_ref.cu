@@ -124,9 +124,8 @@ cudaError_t L_ext_qcount(const ExtractDev* e, int blocks, cudaStream_t st) {
   CLAY_LAUNCH(k_ext_qcount, blocks, kExtractThreads, st, e);
 }
 cudaError_t L_ext_qemit(const ExtractDev* e, int blocks, cudaStream_t st) {
-  CLAY_LAUNCH(k_ext_qemit, blocks, kExtractThreads, st, e);
+  CLAY_LAUNCH(k_ext_qemit, blocks + 1, kExtractThreads, st, e);
 }
-cudaError_t L_ext_finish(const ExtractDev* e, cudaStream_t st) { CLAY_LAUNCH(k_ext_finish, 1, kExtractThreads, st, e); }
 cudaError_t L_build(const BuildDev& b, int tiles, const BrushDev* brushes, int n, cudaStream_t st) {
   CLAY_LAUNCH(k_build, tiles, 256, st, b, brushes, n);
 }

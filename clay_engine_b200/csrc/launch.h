@@ -67,7 +67,6 @@ cudaError_t L_ext_scan(const ExtractDev* e, int which, cudaStream_t st);
 cudaError_t L_ext_emit(const ExtractDev* e, int blocks, cudaStream_t st);
 cudaError_t L_ext_qcount(const ExtractDev* e, int blocks, cudaStream_t st);
 cudaError_t L_ext_qemit(const ExtractDev* e, int blocks, cudaStream_t st);
-cudaError_t L_ext_finish(const ExtractDev* e, cudaStream_t st);
 cudaError_t L_build(const BuildDev& b, int tiles, const BrushDev* brushes, int n, cudaStream_t st);
 cudaError_t L_cell_index(const SceneDev* s, uint32_t* out, int n, cudaStream_t st);
 // Census of a frame's algorithmic work (measurement hooks): out[0] += candidates, out[1] +=

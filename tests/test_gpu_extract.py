@@ -142,3 +142,37 @@ def test_motion_continuity(root, oracle):
     x.destroy()
     field.destroy()
     v.destroy()
+
+
+@pytest.mark.parametrize("res", [2, 7, 63, 64, 65])
+def test_lattice_sizes_are_bit_exact(root, oracle, res):
+    """Lattices of a part of a block, of whole blocks, and on either side of the size from which the counts
+    are scanned by a pass of their own (64^3 points: 1,024 blocks), the slice too small for the larger ones."""
+    import torch
+
+    import clay_engine_b200 as ce
+    from clay_engine_b200 import brushes as B, scenes
+
+    box, lo = 2.6, (-1.3, -1.3, -1.3)
+    vol = ce.SdfVolume(root, resolution=32, worldSize=box, origin=lo, mipLevels=1)
+    vol.build(np.concatenate([B.make_brush("sphere", pos=(0.1, 0.0, 0.0), size=0.7), B.make_brush("box", pos=(0.3, 0.5, 0.2), size=(0.4, 0.3, 0.5), material=1.0)]))
+    d, m = vol.download()
+    cap = 4000
+    parts = torch.zeros(cap * 96, dtype=torch.uint8, device="cuda")
+    bodies = torch.zeros(64, dtype=torch.uint8, device="cuda")
+    x = ce.SurfaceExtractor(root, parts, cap, bodies, 1, ce.volumeField(vol), 0, 0, cap, resolution=res)
+    x.setRegion(lo, box)
+    hp, hb = np.zeros(cap, scenes.PARTICLE_RECORD), np.zeros(1, scenes.BODY_RECORD)
+    of = oracle.make_field([oracle.VolumeData(32, 1, lo, box, 4.0, dist=d, mat=m)])
+    idx, draw_args, counts = oracle.extract(of, hp, hb, res, 0, 0, cap, lo, box)
+    for _ in range(2):
+        x.extract()
+    torch.cuda.synchronize()
+    assert np.array_equal(parts.cpu().numpy(), hp.view(np.uint8).reshape(-1))
+    assert np.array_equal(bodies.cpu().numpy(), hb.view(np.uint8).reshape(-1))
+    tri, draw = x.indices()
+    assert np.array_equal(draw, draw_args) and x.counts() == tuple(int(c) for c in counts)
+    assert np.array_equal(tri.reshape(-1), idx[: int(draw_args[0])])
+    assert res < 7 or counts[0] > 50
+    x.destroy()
+    vol.destroy()
