@@ -317,7 +317,8 @@ struct clay_fluid {
   int G = 0;
   double gorig[3] = {0, 0, 0};
   int mode = CLAY_MODE_FAST;
-  uint32_t parts_scan = 1;
+  // blocks of the cell scan: of a scene by itself, and of one among many
+  uint32_t parts_scan = 1, batch_parts = 1;
   // Device memory.
   std::vector<DevBuf> bufs;
   ParticleDev* parts = nullptr;
@@ -1074,9 +1075,12 @@ int clay_fluid_create(clay_ctx* ctx, const clay_field* world, const clay_fluid_o
   P.damping = static_cast<float>((o.set & CLAY_FLUID_DAMPING) ? o.damping : 0.995);
   P.emit_seed = 1;
   P.contact_depth = static_cast<float>(f->radius * 1.5);
-  // Scan parts: enough blocks that one part covers at most ~32k cells of a full box.
+  // Scan parts, a block each. A scene by itself takes one per 8,192 cells of a full box, since a thin spray fills
+  // the box whatever it holds; in a batch, where the scenes fill the device together and most boxes are small, one
+  // per 32,768 cells that the particles could occupy.
   int64_t cells = static_cast<int64_t>(f->G) * f->G * f->G;
-  f->parts_scan = static_cast<uint32_t>(std::min<int64_t>(kMaxParts, std::max<int64_t>(1, std::min(cells, f->capacity * 4) / 32768)));
+  f->parts_scan = static_cast<uint32_t>(std::min<int64_t>(kMaxParts, std::max<int64_t>(1, cells / 8192)));
+  f->batch_parts = static_cast<uint32_t>(std::min<int64_t>(kMaxParts, std::max<int64_t>(1, std::min(cells, f->capacity * 4) / 32768)));
   const int64_t C = f->capacity;
   if ((rc = f->alloc(&f->parts, C)) || (rc = f->alloc(&f->prm, 1)) || (rc = f->alloc(&f->contacts, 1)) ||
       (rc = f->alloc(&f->gs, 1)) || (rc = f->alloc(&f->hs.key, C)) || (rc = f->alloc(&f->hs.rank, C)) ||
@@ -1631,6 +1635,7 @@ int batch_build(clay_batch* b) {
   for (size_t i = 0; i < b->sims.size(); i++) {
     clay_fluid* f = b->sims[i];
     scenes.push_back(f->hs);
+    scenes.back().parts_scan = f->batch_parts;
     b->max_substeps = std::max(b->max_substeps, f->substeps);
     uint32_t obj = static_cast<uint32_t>(i);
     const clay_bucket_tuning bt = b->tuning_of(f->capacity);
@@ -1648,7 +1653,7 @@ int batch_build(clay_batch* b) {
     }
     int eb = static_cast<int>(std::min<int64_t>(8, (f->capacity + T - 1) / T));
     for (int e = 0; e < eb; e++) we.push_back({obj, 0u, static_cast<uint32_t>(e * T), static_cast<uint32_t>(eb * T)});
-    for (uint32_t p = 0; p < f->parts_scan; p++) wsc.push_back({obj, p, 0u, 0u});
+    for (uint32_t p = 0; p < f->batch_parts; p++) wsc.push_back({obj, p, 0u, 0u});
   }
   std::vector<SplatDev> xs, ss, sp;
   std::vector<Work> wxs, wxr, wss, wsr, wso, wsc2, wtr, wmk;
@@ -2226,7 +2231,7 @@ int clay_batch_step_subset(clay_batch* b, const int32_t* scenes, int n, void* st
   for (int q = 0; q < n; q++) {
     clay_fluid* f = b->sims[scenes[q]];
     if (f->live == 0) continue;
-    for (uint32_t p = 0; p < f->parts_scan; p++) tab.push_back({static_cast<uint32_t>(scenes[q]), p, 0u, 0u});
+    for (uint32_t p = 0; p < f->batch_parts; p++) tab.push_back({static_cast<uint32_t>(scenes[q]), p, 0u, 0u});
   }
   const int n_scan = mark() - o_scan;
   // the splat's tables, and the gather's for the scenes that the device may gather

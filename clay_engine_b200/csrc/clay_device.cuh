@@ -765,6 +765,19 @@ __global__ void k_cell_count(const SceneDev* __restrict__ scenes, const Work* __
   }
 }
 
+// The cells of scan part `part` of [0, n): parts begin at multiples of 4 cells, so that the passes read and
+// write them 16 bytes at a time (a box of 1.4 M mostly empty cells around 1,174 particles took 81 + 162 us a
+// substep, cell by cell in one part).
+__device__ __forceinline__ void scan_part(const SceneDev& S, uint32_t part, uint32_t n, uint32_t& beg, uint32_t& end) {
+  const uint32_t per = max(((n + S.parts_scan - 1) / S.parts_scan + 3u) & ~3u, 4096u);  // a small box: part 0 alone
+  beg = min(part * per, n);
+  end = min(beg + per, n);
+}
+__device__ __forceinline__ uint4 scan_counts(const SceneDev& S, uint32_t c, uint32_t end) {
+  if (c + 4u <= end) return *reinterpret_cast<const uint4*>(S.counts + c);
+  return make_uint4(S.counts[c], c + 1u < end ? S.counts[c + 1u] : 0u, c + 2u < end ? S.counts[c + 2u] : 0u, 0u);
+}
+
 // Cell build, pass 3a: partial sums of the counts of [0, L] split into `parts_scan`
 // parts. Part 0 also resets the box accumulators for the next substep.
 __global__ void k_scan_partial(const SceneDev* __restrict__ scenes, const Work* __restrict__ work, int substep) {
@@ -773,12 +786,15 @@ __global__ void k_scan_partial(const SceneDev* __restrict__ scenes, const Work* 
   if (substep >= S.substeps) return;
   if (work_count(S) == 0) return;
   GridState* gs = S.gs;
-  uint32_t n = gs->L + 1;
-  uint32_t P = S.parts_scan;
-  uint32_t per = (n + P - 1) / P;
-  uint32_t beg = min(w.sub * per, n), end = min(beg + per, n);
+  const uint32_t n = gs->L + 1;
+  uint32_t beg, end;
+  scan_part(S, w.sub, n, beg, end);
+  if (beg >= end) return;  // part 0 always has a cell
   uint32_t s = 0;
-  for (uint32_t c = beg + threadIdx.x; c < end; c += blockDim.x) s += S.counts[c];
+  for (uint32_t c = beg + 4u * threadIdx.x; c < end; c += 4u * blockDim.x) {
+    const uint4 v = scan_counts(S, c, end);
+    s += (v.x + v.y) + (v.z + v.w);
+  }
   s = __reduce_add_sync(0xffffffffu, s);
   __shared__ uint32_t red[32];
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
@@ -801,23 +817,25 @@ __global__ void k_scan_final(const SceneDev* __restrict__ scenes, const Work* __
   if (substep >= S.substeps) return;
   if (work_count(S) == 0) return;
   const GridState* gs = S.gs;
-  uint32_t n = gs->L + 1;
-  uint32_t P = S.parts_scan;
-  uint32_t per = (n + P - 1) / P;
-  uint32_t beg = min(w.sub * per, n), end = min(beg + per, n);
+  const uint32_t n = gs->L + 1;
+  uint32_t beg, end;
+  scan_part(S, w.sub, n, beg, end);
+  if (beg >= end) return;
   __shared__ uint32_t s_off;
   __shared__ uint32_t s_warp[32];
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {
     uint32_t o = 0;
-    for (uint32_t q = 0; q < w.sub; q++) o += gs->part_sum[q];
-    s_off = o;
+    for (uint32_t q = threadIdx.x; q < w.sub; q += 32u) o += gs->part_sum[q];
+    o = __reduce_add_sync(0xffffffffu, o);
+    if (threadIdx.x == 0) s_off = o;
   }
   __syncthreads();
   uint32_t run = s_off;
   const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (uint32_t c0 = beg; c0 < end; c0 += blockDim.x) {
-    uint32_t c = c0 + threadIdx.x;
-    uint32_t v = c < end ? S.counts[c] : 0u;
+  for (uint32_t c0 = beg; c0 < end; c0 += 4u * blockDim.x) {
+    const uint32_t c = c0 + 4u * threadIdx.x;
+    const uint4 q = c < end ? scan_counts(S, c, end) : make_uint4(0u, 0u, 0u, 0u);
+    const uint32_t v = (q.x + q.y) + (q.z + q.w);
     uint32_t x = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -837,16 +855,23 @@ __global__ void k_scan_final(const SceneDev* __restrict__ scenes, const Work* __
     }
     __syncthreads();
     uint32_t before = (wid > 0 ? s_warp[wid - 1] : 0u) + x - v;
-    if (c < end) {
-      S.cell_start[c] = run + before;
-      S.counts[c] = 0u;
+    const uint32_t at = run + before;
+    const uint4 starts = make_uint4(at, at + q.x, at + q.x + q.y, at + q.x + q.y + q.z);
+    if (c + 4u <= end) {
+      *reinterpret_cast<uint4*>(S.cell_start + c) = starts;
+      *reinterpret_cast<uint4*>(S.counts + c) = make_uint4(0u, 0u, 0u, 0u);
+    } else {
+      const uint32_t a[3] = {starts.x, starts.y, starts.z};
+      for (uint32_t k = 0; k < 3 && c + k < end; k++) {
+        S.cell_start[c + k] = a[k];
+        S.counts[c + k] = 0u;
+      }
     }
     uint32_t tot = s_warp[nw - 1];
     __syncthreads();
     run += tot;
   }
-  if (end == n && beg < end && threadIdx.x == 0) S.cell_start[n] = run;
-  if (n == 0 && threadIdx.x == 0 && w.sub == 0) S.cell_start[0] = 0;
+  if (end == n && threadIdx.x == 0) S.cell_start[n] = run;
 }
 
 // Cell build, pass 4: provisional placement.

@@ -286,3 +286,35 @@ def test_upload_far_away_after_stepping_bit_exact(root, oracle):
         assert sim.particleCount == ref.live
         assert_state_equal(sim.download(), ref.parts, sim.particleCount, f"after the spawn, frame {frame}: ")
     sim.destroy()
+
+
+@pytest.mark.parametrize("n, far", [(3, 0.0), (4, 0.35), (700, 2.0), (700, 11.0), (5000, 11.5)])
+def test_scan_of_sparse_boxes_is_bit_exact(root, oracle, n, far):
+    """The cell table of boxes from one cell to the whole grid, most cells empty: parts of the scan of any
+    length modulo four cells, fewer cells than parts; alone and in a batch (fewer parts)."""
+    import clay_engine_b200 as ce
+    from clay_engine_b200.core import PARTICLE_DTYPE
+    from oracle.fluid_frame import OracleFluid
+
+    rng = np.random.default_rng(n)
+    p = np.zeros(n, PARTICLE_DTYPE)
+    p["pos"] = rng.uniform((-far, -min(far, 3.5), -far), (far, far, far), (n, 3)) if far else 0.01 * rng.normal(size=(n, 3))
+    opts = dict(capacity=n, spacing=0.1, radius=0.05, substeps=2, gravity=(0, -9.8, 0), bakeResolution=16, bakeMipLevels=1,
+                bakeBand=2.0, worldSize=24.0, origin=(-12.0, -4.0, -12.0))
+    ref = OracleFluid(oracle, [], **opts)
+    ref.upload(p)
+    sims = [ce.FluidSim(root, None, opts) for _ in range(2)]
+    for s in sims:
+        s.set_mode("reference")
+        s.upload(p)
+    b = ce.Batch(root, sims[1:])
+    for _ in range(2):
+        ref.step()
+        sims[0].step()
+        b.step()
+    for s in sims:
+        g = s.download()
+        for name in ("pos", "vel", "density"):
+            assert np.array_equal(np.ascontiguousarray(g[name]).view(np.uint32), np.ascontiguousarray(ref.parts[name]).view(np.uint32)), name
+    for o in [b] + sims:
+        o.destroy()
