@@ -1246,6 +1246,10 @@ int fluid_substep_plain(clay_fluid* f, cudaStream_t s, int sub) {
   if (f->mode == CLAY_MODE_REFERENCE) {
     CK(L_density_ref(d, nullptr, pb, T, sub, s));
     CK(L_forces_ref(d, nullptr, pb, T, sub, s));
+  } else if (f->live <= kTeamMost) {
+    const int tb = static_cast<int>((f->live + kTeamSize - 1) / kTeamSize);
+    CK(L_density_team(d, nullptr, tb, sub, s));
+    CK(L_forces_team(d, nullptr, tb, sub, s));
   } else {
     CK(L_density_fast(d, nullptr, pb, T, sub, s));
     CK(L_forces_fast(d, nullptr, pb, T, sub, s));

@@ -591,6 +591,12 @@ __device__ __forceinline__ Work get_work_reversed(const Work* work) {
   return w;
 }
 
+// Particles of a block of the team passes (see k_density_team): a table of its own, or blocks of 32.
+__device__ __forceinline__ Work get_team_work(const Work* work) {
+  if (work) return work[blockIdx.x];
+  return {0u, 0u, blockIdx.x * 32u, 32u};
+}
+
 // cellOf (fluid.ts:253-257).
 __device__ __forceinline__ void cell_of(const SceneDev& S, float px, float py, float pz, int& cx, int& cy, int& cz) {
   cx = f2i(floorf((px - S.gorig[0]) * S.inv_h));
@@ -998,6 +1004,20 @@ __device__ __forceinline__ uint32_t local_cell(const SceneDev& S, const BoxInfo&
   return static_cast<uint32_t>(cx - b.x0) + b.bx * (static_cast<uint32_t>(cy - b.y0) + b.by * static_cast<uint32_t>(cz - b.z0));
 }
 
+// What the density pass leaves of particle k: its density, pressure, 1/density and neighbour count, and the
+// neighbour view for the forces pass (svel is not read in this pass): position with 1/density, and beside the
+// velocity the pressure, in fast mode p / rho, so that the forces pass forms a neighbour's
+// (p_i + p_j) / rho_j as one multiply-add, p_i * (1 / rho_j) + p_j / rho_j.
+template <bool kFast>
+__device__ __forceinline__ void density_store(const SceneDev& S, uint32_t k, const float4 me, float rho, uint32_t cnt) {
+  const float stiff = S.prm->stiffness;
+  const float dens = fmaxf(rho, S.rest_floor);
+  const float pres = fmaxf(stiff * (rho - S.rest), 0.0f), inv = __frcp_rn(dens);
+  S.sdp[k] = make_float4(dens, pres, inv, __uint_as_float(cnt));
+  S.spx[k] = make_float4(me.x, me.y, me.z, inv);
+  S.svel[k].w = kFast ? pres * inv : pres;
+}
+
 constexpr int kDensityStage = 3040;  // staged neighbour positions per block (47.5 KB, under the 48 KB static limit)
 
 // density (fluid.ts:333-368). kFast accumulates with Kahan compensation.
@@ -1154,15 +1174,7 @@ __global__ void __launch_bounds__(256, 5) k_density(const SceneDev* __restrict__
     }
   });
   if (kFast) rho = mp6 * __fsub_rn(rho, comp);
-  const float stiff = S.prm->stiffness;
-  const float dens = fmaxf(rho, S.rest_floor);
-  const float pres = fmaxf(stiff * (rho - S.rest), 0.0f), inv = __frcp_rn(dens);
-  S.sdp[k] = make_float4(dens, pres, inv, __uint_as_float(cnt));
-  // the neighbour view of this particle for the forces pass (svel is not read in this pass);
-  // fast mode stores p / rho beside the velocity, so that the forces pass forms a neighbour's
-  // (p_i + p_j) / rho_j as one multiply-add, p_i * (1 / rho_j) + p_j / rho_j
-  S.spx[k] = make_float4(me.x, me.y, me.z, inv);
-  S.svel[k].w = kFast ? pres * inv : pres;
+  density_store<kFast>(S, k, me, rho, cnt);
 }
 
 // integrate (fluid.ts:449-491) of cell-ordered particle k: advance with the new velocity, collide
@@ -1200,6 +1212,69 @@ __device__ __forceinline__ void integrate_particle(const SceneDev& S, const Para
   out.b = make_float4(clx == px ? vx : 0.0f, cly == py ? vy : 0.0f, clz == pz ? vz : 0.0f, mdp.y);
   out.c = make_float4(nvx, nvy, nvz, 0.0f);
   S.parts[S.sorted_id[k]] = out;
+}
+
+// The velocity after the forces (fluid.ts:410-437): pressure and gravity, XSPH viscosity, damping, the speed cap.
+__device__ __forceinline__ void new_velocity(const SceneDev& S, const ParamsDev& P, const float4 mv, const float4 mdp, float fx, float fy,
+                                             float fz, float vsx, float vsy, float vsz, float wsum, float& vx, float& vy, float& vz) {
+  float id = mdp.z;
+  float ax = fx * id + P.gravity[0], ay = fy * id + P.gravity[1], az = fz * id + P.gravity[2];
+  float t = clampf(P.viscosity, 0.0f, 1.0f);
+  float iw = __frcp_rn(wsum);
+  float mx = vsx * iw, my = vsy * iw, mz = vsz * iw;
+  float omt = 1.0f - t;
+  vx = mv.x * omt + mx * t;
+  vy = mv.y * omt + my * t;
+  vz = mv.z * omt + mz * t;
+  vx = (vx + ax * P.dt) * P.damping;
+  vy = (vy + ay * P.dt) * P.damping;
+  vz = (vz + az * P.dt) * P.damping;
+  float speed = len3(vx, vy, vz);
+  if (speed > P.max_speed) {
+    float sc = __fdiv_rn(P.max_speed, speed);
+    vx = vx * sc;
+    vy = vy * sc;
+    vz = vz * sc;
+  }
+}
+
+// Whether cell-ordered particle k is among its own neighbours (the density pass lists it at r = 0): not outside the
+// grid, and not past the bucket of an overfull cell.
+__device__ __forceinline__ bool self_listed(const SceneDev& S, const BoxInfo& b, bool overflow, uint32_t k, int cx, int cy, int cz) {
+  if (cx < 0 || cy < 0 || cz < 0 || cx >= S.G || cy >= S.G || cz >= S.G) return false;
+  if (!overflow) return true;
+  const uint32_t l = static_cast<uint32_t>(cx - b.x0) + b.bx * (static_cast<uint32_t>(cy - b.y0) + b.by * static_cast<uint32_t>(cz - b.z0));
+  return k - S.cell_start[l] < S.bucket;
+}
+
+// Fast mode, one neighbour found in the cells (of a particle with more neighbours than its list holds), in operations
+// that no compiler contracts: k_forces_integrate and k_forces_team add the same terms in the same order, so that a
+// scene's particles come out the same whichever of the two its size selects.
+struct CellPair {
+  float dx, dy, dz, wv, s;  // s: the pressure factor over r, 0 at r = 0
+  __device__ __forceinline__ bool set(const float4 me, const float4 o, float h2) {
+    dx = __fsub_rn(me.x, o.x);
+    dy = __fsub_rn(me.y, o.y);
+    dz = __fsub_rn(me.z, o.z);
+    s = __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));  // the squared length, for now
+    return s < h2;
+  }
+  __device__ __forceinline__ void weigh(float inv, float p_rho, float mp, float h, float h2, float half_mass_spiky) {
+    const float r2 = s, w0 = __fsub_rn(h2, r2);
+    wv = __fmul_rn(__fmul_rn(w0, w0), w0);
+    const float irs = rsqrtf(r2), r = __fmul_rn(r2, irs), hr = __fsub_rn(h, r);
+    s = r > 1e-6f ? __fmul_rn(__fmul_rn(half_mass_spiky, __fmaf_rn(mp, inv, p_rho)), __fmul_rn(__fmul_rn(hr, hr), irs)) : 0.0f;
+  }
+};
+__device__ __forceinline__ void add_pair(float dx, float dy, float dz, float wv, float s, float ox, float oy, float oz, float& fx,
+                                         float& fy, float& fz, float& vsx, float& vsy, float& vsz, float& wsum) {
+  vsx = __fmaf_rn(ox, wv, vsx);
+  vsy = __fmaf_rn(oy, wv, vsy);
+  vsz = __fmaf_rn(oz, wv, vsz);
+  wsum = __fadd_rn(wsum, wv);
+  fx = __fmaf_rn(-dx, s, fx);
+  fy = __fmaf_rn(-dy, s, fy);
+  fz = __fmaf_rn(-dz, s, fz);
 }
 
 // forces (fluid.ts:370-439) fused with integrate (fluid.ts:449-491). The neighbour pass
@@ -1301,7 +1376,7 @@ __global__ void __launch_bounds__(256, kSplit ? 5 : 4) k_forces_integrate(const 
   if (cnt <= kMaxNbr) {
     const uint4* __restrict__ nl = S.nbr + k;
     const uint32_t stride = S.capacity;
-    if (kFast) {  // the particle's own entry brings its term
+    if (kFast && self_listed(S, b, overflow, k, cx, cy, cz)) {  // the particle's own entry brings its term
       vsx = 0.0f;
       vsy = 0.0f;
       vsz = 0.0f;
@@ -1338,26 +1413,20 @@ __global__ void __launch_bounds__(256, kSplit ? 5 : 4) k_forces_integrate(const 
     uint32_t j = 0;
     for (; j + 4u <= cnt; j += 4) slot(j, 4u);
     if (j < cnt) slot(j, cnt - j);
+  } else if constexpr (kFast) {
+    for_neighbours(S, b, overflow, cx, cy, cz, [&](uint32_t q) {
+      const float4 o = __ldg(spx + q);
+      CellPair c;
+      if (q == k || !c.set(me, o, h2)) return;
+      const float4 ov = __ldg(svel + q);
+      c.weigh(o.w, ov.w, mp, h, h2, half_mass_spiky);
+      add_pair(c.dx, c.dy, c.dz, c.wv, c.s, ov.x, ov.y, ov.z, fx, fy, fz, vsx, vsy, vsz, wsum);
+    });
   } else {
     for_neighbours(S, b, overflow, cx, cy, cz, pair);
   }
-  float id = mdp.z;
-  float ax = fx * id + P.gravity[0], ay = fy * id + P.gravity[1], az = fz * id + P.gravity[2];
-  float t = clampf(P.viscosity, 0.0f, 1.0f);
-  float iw = __frcp_rn(wsum);
-  float mx = vsx * iw, my = vsy * iw, mz = vsz * iw;
-  float omt = 1.0f - t;
-  float vx = mv.x * omt + mx * t, vy = mv.y * omt + my * t, vz = mv.z * omt + mz * t;
-  vx = (vx + ax * P.dt) * P.damping;
-  vy = (vy + ay * P.dt) * P.damping;
-  vz = (vz + az * P.dt) * P.damping;
-  float speed = len3(vx, vy, vz);
-  if (speed > P.max_speed) {
-    float sc = __fdiv_rn(P.max_speed, speed);
-    vx = vx * sc;
-    vy = vy * sc;
-    vz = vz * sc;
-  }
+  float vx, vy, vz;
+  new_velocity(S, P, mv, mdp, fx, fy, fz, vsx, vsy, vsz, wsum, vx, vy, vz);
   if constexpr (kSplit) {
     // the integrate pass runs as its own launch: the new velocity waits in the first entry of
     // this particle's neighbour list, which no other particle reads
@@ -1381,6 +1450,196 @@ __global__ void __launch_bounds__(256) k_integrate(const SceneDev* __restrict__ 
   const float4 v = reinterpret_cast<const float4*>(S.nbr)[k];
   integrate_particle(S, *S.prm, k, S.spos[k], S.sdp[k], v.x, v.y, v.z);
 }
+
+#ifdef CLAY_TEAM_PASSES
+// The neighbour passes of few particles (fast mode): kTeam lanes share a particle. A thread walks some 290
+// candidates of a dense particle one after another, about 200 cycles each whatever runs beside it, so a scene
+// that does not fill the device takes as long as one thread: 4,096 particles 31 us (density) and 18 us
+// (forces) a substep, on 16 of 148 SMs. With eight lanes a particle its loads and tests are an eighth as long a
+// chain, and the sums are added up in the thread's order, so the results are the same bits: a frame 167.7 -> 139.1.
+// Above kTeamMost particles the lanes' shared overhead costs more than the shorter chain saves (dense frames of
+// 12,000, 20,000, 24,000 and 48,000: 144, 168, 184 and 259 us with teams, 170, 176, 175 and 197 with a thread each).
+constexpr uint32_t kTeam = 8, kTeamBlock = 256, kTeamParticles = kTeamBlock / kTeam;
+
+// The 27 cells' candidates of the warp's particles (`valid` lanes), in the order of for_neighbours, kTeam at a
+// time: f(q, ok) for all lanes of the warp together, with this lane's candidate where ok.
+template <class F>
+__device__ __forceinline__ void team_candidates(const SceneDev& S, const BoxInfo& b, bool overflow, bool valid, int cx, int cy,
+                                                int cz, F&& f) {
+  const uint32_t sub = threadIdx.x % kTeam;
+  const int G = S.G;
+  cx = min(max(cx, -2), G + 1);
+  cy = min(max(cy, -2), G + 1);
+  cz = min(max(cz, -2), G + 1);
+  const int x1b = b.x0 + static_cast<int>(b.bx) - 1, y1b = b.y0 + static_cast<int>(b.by) - 1, z1b = b.z0 + static_cast<int>(b.bz) - 1;
+  const int xl = max(cx - 1, b.x0), xh = min(cx + 1, x1b);
+  valid = valid && b.L != 0 && xl <= xh;
+  // the rows' ranges, a row per lane of the team (the ninth again by the first)
+  auto row_range = [&](uint32_t r, uint32_t& s, uint32_t& e, uint32_t& l) {
+    const int z = cz + static_cast<int>(r / 3) - 1, y = cy + static_cast<int>(r % 3) - 1;
+    s = e = l = 0;
+    if (!valid || z < b.z0 || z > z1b || y < b.y0 || y > y1b) return;
+    l = b.bx * (static_cast<uint32_t>(y - b.y0) + b.by * static_cast<uint32_t>(z - b.z0)) + static_cast<uint32_t>(xl - b.x0);
+    s = __ldg(S.cell_start + l);
+    e = __ldg(S.cell_start + l + static_cast<uint32_t>(xh - xl) + 1u);
+  };
+  auto walk = [&](uint32_t s, uint32_t e) {
+    for (uint32_t q = s + sub; __any_sync(0xffffffffu, q < e); q += kTeam) f(q, q < e);
+  };
+  uint32_t s0, e0, l0, s8, e8, l8;
+  row_range(sub, s0, e0, l0);
+  row_range(8, s8, e8, l8);
+#pragma unroll 1
+  for (uint32_t r = 0; r < 9; r++) {
+    const uint32_t s = r < 8 ? __shfl_sync(0xffffffffu, s0, r, kTeam) : s8, e = r < 8 ? __shfl_sync(0xffffffffu, e0, r, kTeam) : e8;
+    if (!overflow) {
+      walk(s, e);
+      continue;
+    }
+    // a cell over its bucket keeps its first `bucket` particles: cell by cell
+    const uint32_t l = r < 8 ? __shfl_sync(0xffffffffu, l0, r, kTeam) : l8;
+    for (uint32_t c = 0; c < 3; c++) {
+      const bool in = e > s && c <= static_cast<uint32_t>(xh - xl);
+      const uint32_t a = in ? S.cell_start[l + c] : 0u, z = in ? S.cell_start[l + c + 1u] : 0u;
+      walk(a, a + min(z - a, S.bucket));
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kTeamBlock) k_density_team(const SceneDev* __restrict__ scenes, const Work* __restrict__ work,
+                                                              int substep) {
+  const Work w = get_team_work(work);
+  const SceneDev& S = scenes[w.obj];
+  if (substep >= S.substeps) return;
+  const uint32_t sub = threadIdx.x % kTeam, slot = threadIdx.x / kTeam, k = w.first + slot;
+  const bool valid = k < work_count(S) && slot < w.n;
+  const BoxInfo b = box_from_state(S.gs);
+  const bool overflow = S.gs->overflow != 0u;
+  const float4 me = valid ? S.spos[k] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  int cx, cy, cz;
+  cell_of(S, me.x, me.y, me.z, cx, cy, cz);
+  const float h2 = S.h2;
+  float rho = 0.0f, comp = 0.0f;
+  const float4* __restrict__ spos = S.spos;
+  uint32_t* __restrict__ nl = reinterpret_cast<uint32_t*>(S.nbr + k);
+  const uint32_t stride = 4u * S.capacity, shift = threadIdx.x & 31u & ~(kTeam - 1u);
+  uint32_t cnt = 0;
+  team_candidates(S, b, overflow, valid, cx, cy, cz, [&](uint32_t q, bool ok) {
+    const float4 o = __ldg(spos + (ok ? q : 0u));
+    const float dx = me.x - o.x, dy = me.y - o.y, dz = me.z - o.z;
+    const float r2 = (dx * dx + dy * dy) + dz * dz;
+    const bool take = ok && r2 < h2;
+    // the list in visiting order: the team's lanes hold consecutive candidates
+    const uint32_t mine = (__ballot_sync(0xffffffffu, take) >> shift) & ((1u << kTeam) - 1u);
+    const float wv = h2 - r2, term = (wv * wv) * wv;
+    if (take) {
+      const uint32_t j = cnt + __popc(mine & ((1u << sub) - 1u));
+      if (j < kMaxNbr) nl[(j >> 2) * stride + (j & 3u)] = q;
+    }
+    cnt += __popc(mine);
+    // the terms in the same order, one after another in every lane: the sum of k_density, bit for bit
+    for (uint32_t left = mine; __any_sync(0xffffffffu, left != 0u); left &= left - 1u) {
+      const float next = __shfl_sync(0xffffffffu, term, left ? __ffs(left) - 1 : 0, kTeam);
+      if (left) {
+        const float y = __fsub_rn(next, comp), t = __fadd_rn(rho, y);
+        comp = __fsub_rn(__fsub_rn(t, rho), y);
+        rho = t;
+      }
+    }
+  });
+  if (!valid || sub != 0) return;
+  density_store<true>(S, k, me, S.mass_poly6 * __fsub_rn(rho, comp), cnt);
+}
+
+__global__ void __launch_bounds__(kTeamBlock) k_forces_team(const SceneDev* __restrict__ scenes, const Work* __restrict__ work,
+                                                             int substep) {
+  const Work w = get_team_work(work);
+  const SceneDev& S = scenes[w.obj];
+  if (substep >= S.substeps) return;
+  const uint32_t sub = threadIdx.x % kTeam, slot = threadIdx.x / kTeam, k = w.first + slot;
+  const bool valid = k < work_count(S) && slot < w.n;
+  const ParamsDev& P = *S.prm;
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const float4 me = valid ? S.spos[k] : zero, mv = valid ? S.svel[k] : zero, mdp = valid ? S.sdp[k] : zero;
+  const float h2 = S.h2, h = S.h, half_mass_spiky = (S.mass * 0.5f) * S.spiky, mp = mdp.y;
+  const BoxInfo b = box_from_state(S.gs);
+  const bool overflow = S.gs->overflow != 0u;
+  int cx, cy, cz;
+  cell_of(S, me.x, me.y, me.z, cx, cy, cz);
+  const uint32_t cnt = valid ? __float_as_uint(mdp.w) : 0u;
+  float fx = 0.0f, fy = 0.0f, fz = 0.0f, vsx = 0.0f, vsy = 0.0f, vsz = 0.0f, wsum = 0.0f;
+  if (cnt > kMaxNbr || !self_listed(S, b, overflow, k, cx, cy, cz)) {
+    vsx = mv.x * S.h6;
+    vsy = mv.y * S.h6;
+    vsz = mv.z * S.h6;
+    wsum = S.h6;
+  }
+  const uint32_t* __restrict__ nl = reinterpret_cast<const uint32_t*>(S.nbr + k);
+  const uint32_t stride = 4u * S.capacity, listed = cnt <= kMaxNbr ? cnt : 0u;
+  for (uint32_t j0 = 0; __any_sync(0xffffffffu, j0 < listed); j0 += kTeam) {
+    // a neighbour a lane, as accum_listed of k_forces_integrate
+    const uint32_t j = j0 + sub;
+    float dx = 0.0f, dy = 0.0f, dz = 0.0f, wv = 0.0f, t = 0.0f;
+    float4 ov = zero;
+    if (j < listed) {
+      const uint32_t q = __ldg(nl + ((j >> 2) * stride + (j & 3u)));
+      const float4 o = __ldg(S.spx + q);
+      ov = __ldg(S.svel + q);
+      dx = me.x - o.x;
+      dy = me.y - o.y;
+      dz = me.z - o.z;
+      const float r2 = (dx * dx + dy * dy) + dz * dz;
+      const float w0 = h2 - r2;
+      wv = (w0 * w0) * w0;
+      if (r2 > 1e-12f) {  // r > 1e-6
+        const float irs = rsqrtf(r2);
+        const float hr = h - r2 * irs;
+        t = half_mass_spiky * fmaf(mp, o.w, ov.w) * ((hr * hr) * irs);
+      }
+    }
+    // added up in the list's order in every lane: the sums of k_forces_integrate, bit for bit
+#pragma unroll
+    for (uint32_t u = 0; u < kTeam; u++) {
+      auto from = [&](float x) { return __shfl_sync(0xffffffffu, x, u, kTeam); };
+      const float nw = from(wv), nt = from(t), ox = from(ov.x), oy = from(ov.y), oz = from(ov.z), ex = from(dx), ey = from(dy), ez = from(dz);
+      if (j0 + u < listed) {
+        vsx = vsx + ox * nw;
+        vsy = vsy + oy * nw;
+        vsz = vsz + oz * nw;
+        wsum = wsum + nw;
+        fx = fx - ex * nt;
+        fy = fy - ey * nt;
+        fz = fz - ez * nt;
+      }
+    }
+  }
+  if (__any_sync(0xffffffffu, cnt > kMaxNbr)) {  // more neighbours than the list holds: the cells again
+    const uint32_t shift = threadIdx.x & 31u & ~(kTeam - 1u);
+    team_candidates(S, b, overflow, cnt > kMaxNbr, cx, cy, cz, [&](uint32_t q, bool ok) {
+      const float4 o = __ldg(S.spx + (ok ? q : 0u));
+      CellPair c;
+      const bool take = c.set(me, o, h2) && ok && q != k;
+      float4 ov = zero;
+      if (take) {
+        ov = __ldg(S.svel + q);
+        c.weigh(o.w, ov.w, mp, h, h2, half_mass_spiky);
+      }
+      uint32_t left = (__ballot_sync(0xffffffffu, take) >> shift) & ((1u << kTeam) - 1u);
+      for (; __any_sync(0xffffffffu, left != 0u); left &= left - 1u) {
+        const int u = left ? __ffs(left) - 1 : 0;
+        auto from = [&](float x) { return __shfl_sync(0xffffffffu, x, u, kTeam); };
+        const float ex = from(c.dx), ey = from(c.dy), ez = from(c.dz), nw = from(c.wv), ns = from(c.s), ox = from(ov.x), oy = from(ov.y),
+                    oz = from(ov.z);
+        if (left) add_pair(ex, ey, ez, nw, ns, ox, oy, oz, fx, fy, fz, vsx, vsy, vsz, wsum);
+      }
+    });
+  }
+  if (!valid || sub != 0) return;
+  float vx, vy, vz;
+  new_velocity(S, P, mv, mdp, fx, fy, fz, vsx, vsy, vsz, wsum, vx, vy, vz);
+  integrate_particle(S, P, k, me, mdp, vx, vy, vz);
+}
+#endif  // CLAY_TEAM_PASSES
 
 // ---------------------------------------------------------------------------------------
 // SplatField bake (splat.ts:200-276).

@@ -2,6 +2,7 @@
 // the density sum is compensated. Compiled with -fmad=true.
 #define CLAY_DEFINE_KERNELS
 #define CLAY_ONLY_NEIGHBOUR_PASSES
+#define CLAY_TEAM_PASSES
 #include "launch.h"
 
 namespace clay {
@@ -23,6 +24,17 @@ cudaError_t L_forces_fast(const SceneDev* s, const Work* w, int blocks, int thre
   } else {
     k_forces_integrate<true, false><<<blocks, threads, 0, st>>>(s, w, sub);
   }
+  count_launch();
+  return cudaPeekAtLastError();
+}
+
+cudaError_t L_density_team(const SceneDev* s, const Work* w, int blocks, int sub, cudaStream_t st) {
+  k_density_team<<<blocks, kTeamBlock, 0, st>>>(s, w, sub);
+  count_launch();
+  return cudaPeekAtLastError();
+}
+cudaError_t L_forces_team(const SceneDev* s, const Work* w, int blocks, int sub, cudaStream_t st) {
+  k_forces_team<<<blocks, kTeamBlock, 0, st>>>(s, w, sub);
   count_launch();
   return cudaPeekAtLastError();
 }

@@ -42,6 +42,9 @@ cudaError_t L_density_fast(const SceneDev* s, const Work* w, int blocks, int thr
                            int variant = kDensityVariant);
 cudaError_t L_forces_fast(const SceneDev* s, const Work* w, int blocks, int threads, int sub, cudaStream_t st,
                           bool split = false);
+// Fast mode, few particles: `blocks` of 32 particles, eight lanes each.
+cudaError_t L_density_team(const SceneDev* s, const Work* w, int blocks, int sub, cudaStream_t st);
+cudaError_t L_forces_team(const SceneDev* s, const Work* w, int blocks, int sub, cudaStream_t st);
 // `blocks_y` = mip levels when w == nullptr.
 // acc_voxels: size of the shared-memory minimum tile (dynamic shared memory, 4 B per voxel).
 cudaError_t L_splat(const SplatDev* d, const Work* w, int blocks, int blocks_y, uint32_t acc_voxels, cudaStream_t st);
@@ -76,6 +79,8 @@ cudaError_t L_census_splat(const SplatDev* d, int blocks, int mips, unsigned lon
 cudaError_t L_gather_contacts(const SceneDev* s, int n, ContactsDev* out, cudaStream_t st);
 cudaError_t L_field_query(const FieldDev* f, const float* pts, int n, float* sxy, float* nrm, cudaStream_t st);
 
+constexpr int kTeamSize = 32;         // particles per block of the team passes
+constexpr int64_t kTeamMost = 20480;   // particles stepped together up to which they are taken (see k_density_team)
 constexpr int kScanThreads = 1024;
 constexpr int kSplatThreads = 32 * kSplatWarps;
 constexpr int kResolveThreads = 256;

@@ -318,3 +318,33 @@ def test_scan_of_sparse_boxes_is_bit_exact(root, oracle, n, far):
             assert np.array_equal(np.ascontiguousarray(g[name]).view(np.uint32), np.ascontiguousarray(ref.parts[name]).view(np.uint32)), name
     for o in [b] + sims:
         o.destroy()
+
+
+@pytest.mark.parametrize("n, spacing, bucket", [(1, 0.1, 64), (31, 0.1, 64), (33, 0.1, 64), (1000, 0.07, 64), (3000, 0.1, 6),
+                                                (3000, 0.4, 64),
+                                                (20480, 0.1, 64), (20481, 0.1, 64), (25000, 0.1, 6)])
+def test_fast_neighbour_passes_by_size(root, n, spacing, bucket):
+    """One fast frame against a reference-mode one from the same state, within the fast mode's bounds (2e-5 of the
+    scale for positions and density, 1e-4 velocities, 2e-4 pressure): particles on either side of a block of the
+    team passes and of the size up to which they are taken, more neighbours than a list holds, overfull cells (some
+    particles are then not among their own neighbours, nor are those outside the grid)."""
+    import clay_engine_b200 as ce
+    from clay_engine_b200 import scenes
+
+    p = scenes.lattice_block(n, spacing, (0.2, 1.0, -0.3), n)
+    p["vel"] = np.random.default_rng(n).normal(0, 0.3, (n, 3))
+    if n > 100:
+        p["pos"][::97, 1] += 40.0
+    out = []
+    for mode in ("reference", "fast"):
+        s = ce.FluidSim(root, None, dict(capacity=n + 7, spacing=0.1, radius=0.05, substeps=1, bucket=bucket, bakeResolution=16,
+                                         bakeMipLevels=1, worldSize=24.0, origin=(-12.0, -4.0, -12.0)))
+        s.set_mode(mode)
+        s.upload(p)
+        s.step()
+        out.append(s.download())
+        s.destroy()
+    ref, fast = out
+    for name, tol in (("pos", 2e-5), ("density", 2e-5), ("vel", 1e-4), ("nvel", 1e-4), ("pressure", 2e-4)):
+        scale = max(float(np.abs(ref[name]).max()), 1e-3)
+        assert np.isfinite(ref[name]).all() and np.abs(ref[name] - fast[name]).max() <= tol * scale, name
