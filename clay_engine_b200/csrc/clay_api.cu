@@ -64,6 +64,7 @@ namespace {
   } while (0)
 
 constexpr int TILE = 8;
+constexpr int64_t kDiscsLeast = 16, kDiscBlocks = 148 * 3;  // discs per block at least, blocks wanted at most
 constexpr int kMaxBrushes = 256;  // one per thread of the build's cull
 constexpr int kMaxResolution = 4096;  // 4096^3 voxels per level: far beyond device memory, far below int64 overflow
 
@@ -605,8 +606,13 @@ int splat_bake(clay_splat* s, cudaStream_t st, const SceneDev* scene, int64_t it
   }
   const SplatDev* d = scene ? s->d_plain : s->d;
   if (n > 0) {
-    int blocks = static_cast<int>((n + kSplatThreads - 1) / kSplatThreads);
-    CK(L_splat(d, nullptr, blocks, s->mips, s->cloud.normals ? kSplatAccVoxelsDiscs : kSplatAccVoxels, st));
+    // a small disc cloud in blocks of fewer particles, until they fill the device (see k_splat)
+    int64_t per = kSplatThreads;
+    if (s->cloud.normals)
+      while (per > kDiscsLeast && (n + per - 1) / per * s->mips < kDiscBlocks) per /= 2;
+    int blocks = static_cast<int>((n + per - 1) / per);
+    CK(L_splat(d, nullptr, blocks, s->mips, s->cloud.normals ? kSplatAccVoxelsDiscs : kSplatAccVoxels, st,
+               static_cast<uint32_t>(per)));
   }
   int64_t quads = (s->vol->total + 3) / 4;
   int rblocks = static_cast<int>((quads + kResolveThreads - 1) / kResolveThreads);

@@ -1761,14 +1761,17 @@ __device__ __forceinline__ void splat_block(const SplatDev& D, const Work w, flo
   __shared__ unsigned long long s_cost;
   __shared__ uint32_t s_woff[kSplatWarps];
   __shared__ uint32_t s_nlive;
-  const uint32_t idx = w.first + threadIdx.x;
   const bool has_n = D.nrm != nullptr;
+  // A block of fewer than 256 discs spreads them over its warps (each walks its own one after another); spheres keep
+  // their order, which the tile walk's slices follow.
+  const uint32_t li = has_n && w.n < 32u * kSplatWarps ? static_cast<uint32_t>(lane * kSplatWarps + wid) : threadIdx.x;
+  const uint32_t idx = w.first + li;
   const float voxel = D.voxel[m], bw = D.bw[m], reach = D.reach[m], inv_voxel = D.inv_voxel[m], radius = D.radius;
   const int R = D.r[m];
   const int last = R - 1;
   const long long off = D.off[m];
   uint32_t i = 0;
-  bool live = (threadIdx.x < w.n) && cloud_live(D, idx, i);
+  bool live = (li < w.n) && cloud_live(D, idx, i);
   float px = 0, py = 0, pz = 0, nx = 0, ny = 0, nz = 0;
   int lx = 0, ly = 0, lz = 0, hx = -1, hy = -1, hz = -1;
   if (live) {
@@ -2524,9 +2527,16 @@ __device__ __forceinline__ void resolve_block(const SplatDev& D, const Work w) {
 }
 
 #ifndef CLAY_ONLY_NEIGHBOUR_PASSES
+// `per`: particles per block where there is no work table. A small disc cloud takes fewer than 256, so that its
+// blocks fill the device: a particle's walk is a chain of its own, and a warp of a full block makes 32 of them one after
+// another (a clay body of 3,800 discs on 30 blocks: 204 us).
 __global__ void __launch_bounds__(32 * kSplatWarps, 4) k_splat(const SplatDev* __restrict__ splats, const Work* __restrict__ work,
-                                                             uint32_t acc_cap) {
-  const Work w = get_work_reversed(work);
+                                                             uint32_t acc_cap, uint32_t per) {
+  Work w = get_work_reversed(work);
+  if (!work) {
+    w.first = (gridDim.x - 1u - blockIdx.x) * per;
+    w.n = per;
+  }
   const SplatDev& D = splats[w.obj];
   if (bake_gathers(D)) return;
   splat_block(D, w, D.vp->origin[0], D.vp->origin[1], D.vp->origin[2], acc_cap);

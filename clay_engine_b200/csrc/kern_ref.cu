@@ -64,7 +64,7 @@ cudaError_t L_forces_ref(const SceneDev* s, const Work* w, int blocks, int threa
   count_launch();
   return cudaPeekAtLastError();
 }
-cudaError_t L_splat(const SplatDev* d, const Work* w, int blocks, int blocks_y, uint32_t acc_voxels, cudaStream_t st) {
+cudaError_t L_splat(const SplatDev* d, const Work* w, int blocks, int blocks_y, uint32_t acc_voxels, cudaStream_t st, uint32_t per) {
   // The splat's shared memory exceeds the default per-block limit; the opt-in is a property
   // of the function on each device, so it is set once per device (from any thread).
   constexpr int kDevices = 64;
@@ -79,7 +79,7 @@ cudaError_t L_splat(const SplatDev* d, const Work* w, int blocks, int blocks_y, 
     if (dev >= 0 && dev < kDevices) attr_set[dev].store(true, std::memory_order_release);
   }
   dim3 g(blocks, w ? 1 : blocks_y);
-  k_splat<<<g, kSplatThreads, acc_voxels * sizeof(uint32_t), st>>>(d, w, acc_voxels);
+  k_splat<<<g, kSplatThreads, acc_voxels * sizeof(uint32_t), st>>>(d, w, acc_voxels, per);
   count_launch();
   return cudaPeekAtLastError();
 }
