@@ -64,7 +64,7 @@ namespace {
   } while (0)
 
 constexpr int TILE = 8;
-constexpr int64_t kDiscsLeast = 16, kDiscBlocks = 148 * 3;  // discs per block at least, blocks wanted at most
+constexpr int64_t kDiscsLeast = 16, kDiscBlocks = 148 * 8;  // discs per block at least, blocks wanted at most
 constexpr int kMaxBrushes = 256;  // one per thread of the build's cull
 constexpr int kMaxResolution = 4096;  // 4096^3 voxels per level: far beyond device memory, far below int64 overflow
 
@@ -586,6 +586,14 @@ void free_splat(clay_splat* s) {
 // Chunks of 8^3 voxels over all levels, in blocks of the mark pass.
 int mark_blocks(const clay_splat* s) { return static_cast<int>((s->vol->total / 512 + kMarkChunks - 1) / kMarkChunks); }
 
+// Discs per block of the splat, given the blocks that so many make.
+template <class Blocks>
+int64_t discs_per_block(Blocks&& blocks) {
+  int64_t per = kSplatThreads;
+  while (per > kDiscsLeast && blocks(per) < kDiscBlocks) per /= 2;
+  return per;
+}
+
 // Blocks over the cloud's iteration space for every mip (plain bake), of a fluid (`scene`) in cell
 // order; a large fluid is gathered.
 int splat_bake(clay_splat* s, cudaStream_t st, const SceneDev* scene, int64_t iter_n) {
@@ -607,9 +615,7 @@ int splat_bake(clay_splat* s, cudaStream_t st, const SceneDev* scene, int64_t it
   const SplatDev* d = scene ? s->d_plain : s->d;
   if (n > 0) {
     // a small disc cloud in blocks of fewer particles, until they fill the device (see k_splat)
-    int64_t per = kSplatThreads;
-    if (s->cloud.normals)
-      while (per > kDiscsLeast && (n + per - 1) / per * s->mips < kDiscBlocks) per /= 2;
+    const int64_t per = s->cloud.normals ? discs_per_block([&](int64_t p) { return (n + p - 1) / p * s->mips; }) : kSplatThreads;
     int blocks = static_cast<int>((n + per - 1) / per);
     CK(L_splat(d, nullptr, blocks, s->mips, s->cloud.normals ? kSplatAccVoxelsDiscs : kSplatAccVoxels, st,
                static_cast<uint32_t>(per)));
@@ -1693,10 +1699,16 @@ int batch_build(clay_batch* b) {
     for (size_t i = 0; i < all.size(); i++) all[i] = static_cast<int>(i);
     b->gather = b->gather && batch_list(b, all).items;  // clay_batch_profile steps them in one lane
   }
+  const int64_t disc_block = discs_per_block([&](int64_t p) {  // the bodies of the batch together
+    int64_t n = 0;
+    for (const clay_splat* x : b->extra) n += (x->cloud.capacity + p - 1) / p * x->mips;
+    return n;
+  });
   for (size_t i = 0; i < b->extra.size(); i++) {
     xs.push_back(b->extra[i]->h);
     xs.back().order = nullptr;
-    add_splat_work(wxs, wxr, static_cast<uint32_t>(i), b->extra[i], b->extra[i]->cloud.capacity, kSplatThreads);
+    add_splat_work(wxs, wxr, static_cast<uint32_t>(i), b->extra[i], b->extra[i]->cloud.capacity,
+                   b->extra[i]->cloud.normals ? static_cast<int>(disc_block) : kSplatThreads);
   }
   for (size_t i = 0; i < b->sims.size(); i++) {
     clay_splat* s = b->sims[i]->surface;
