@@ -475,7 +475,7 @@ def measure_next_rows(root, stream, threads):
     out["solver"] = {"workload": f"86 bodies x {len(shell)} particles, 2 substeps, 2 rotation iterations",
                      "value": npart / (ms / 1e3), "unit": "particle-steps/s", "ms_per_step": ms,
                      "achieved_gbs": npart * 2 * per / (ms / 1e3) / 1e9, "bytes_per_particle_substep": per,
-                     "launches_per_step": 8,
+                     "launches_per_step": 5,
                      "cpu_baseline": {"value": len(sp) / cs, "unit": "particle-steps/s", "cores": 1, "kind": "port",
                                       "sample": f"8 of the bodies ({len(sp)} particles), 1 step"}}
     solver.destroy()
@@ -668,10 +668,8 @@ BYTES_PER_PARTICLE = {
     "density": 16 + 16 + 16 + 4,  # pos in; density record, neighbour view (pos, 1/density), pressure out
     "forces_integrate": 16 + 16 + 16 + 4 + 48,  # pos, vel, density record, id in; particle record out
 }
-# DRAM bytes (read + written) per particle of one k_splat launch over the fluid surfaces (3
-# levels), from one ncu capture of that launch in the 128-scene batch (dram__bytes_read.sum +
-# dram__bytes_write.sum): 107,473,408 + 5,515,008 bytes for 1,940,550 particles.
-SPLAT_TRAFFIC_PER_PARTICLE = (107473408 + 5515008) / 1940550
+# The launches of the fluid surfaces' bake: a dense scene of a large batch is gathered, the others splatted.
+BAKE_PHASES = ("splat", "resolve", "bake_sort", "bake_scatter", "bake_tree", "bake_mark", "bake_gather")
 
 
 def main():
@@ -831,39 +829,31 @@ def main():
         acc += c["accepted"]
         pairs += c["splat_pairs"]
     body_pairs = sum(b.census(stream) for b in bodies)
-    # algorithmic bytes of the bake: each (particle, level) reads its 16-byte position once; each
-    # voxel the bake lowers is read and written once in the key grid (8 B)
-    touched = 0
-    for s in sims:
-        d, _ = s.surface.volume.download()
-        touched += int((d != 0x3C00).sum())
-    mips = sims[0].surface.volume.mipLevels if sims else 0
+    # algorithmic bytes of the bake: each particle's 16-byte position read once, each voxel's f16 distance written once
     n_sims = len(sims)
-    splat_bytes = 16 * particles * mips + 8 * touched
-    # ---- roofline of the dominant kernel, k_splat (its fluid-surface launch "splat": the
-    # SplatField bake of every fluid), from the per-launch event times of one frame
+    splat_bytes = 16 * particles + 2 * sum(s.surface.volume.totalVoxels for s in sims)
+    # ---- roofline of the fluid surfaces' bake (the SplatField bake of every fluid, its launches together), from the
+    # per-launch event times of one frame
     peak, peak_kind = load_peaks()
     # FP32 issue peak at the clock seen during the timed frames: 148 SMs x 128 FP32 lanes
     mhz = clk.get("sm_mhz") or clk.get("sm_max_mhz") or 1965.0
     sms = torch.cuda.get_device_properties(local).multi_processor_count
     lane_peak = sms * 128 * mhz * 1e6
-    splat_ms, splat_launches = prof.get("splat", (None, 0))
-    roof = {"bound": "hbm", "kernel": "k_splat (fluid surfaces)", "achieved": None, "peak": peak, "unit": "GB/s",
+    splat_ms = sum(prof[k][0] for k in BAKE_PHASES if k in prof) or None
+    roof = {"bound": "hbm", "kernel": "fluid surface bake (k_bake_gather and its passes, k_splat)", "achieved": None, "peak": peak, "unit": "GB/s",
             "frac": None, "traffic": None, "peak_source": peak_kind}
     if splat_ms:
-        avg_ms = splat_ms / splat_launches
-        achieved = splat_bytes / (avg_ms / 1000) / 1e9
+        achieved = splat_bytes / (splat_ms / 1000) / 1e9
         roof.update({"achieved": round(achieved, 2), "frac": achieved / peak,
-                     "traffic": SPLAT_TRAFFIC_PER_PARTICLE * particles,
-                     "algorithmic_bytes_per_launch": splat_bytes, "avg_launch_ms": round(avg_ms, 4)})
+                     "algorithmic_bytes_per_launch": splat_bytes, "avg_launch_ms": round(splat_ms, 4)})
     # compute roofline (the kernels are issue-bound): algorithmic FP32 operations of the
-    # reference's work per second against the FP32 lane-issue peak. k_splat: 9 per in-band pair
+    # reference's work per second against the FP32 lane-issue peak. The bake: 9 per in-band pair
     # (3 sub, 3 mul, 2 add, 1 compare); k_density: 9 per candidate + 13 per accepted pair (the
     # kernel term and the sum), over both substeps (the census counts the last one)
     comp = {"unit": "FP32 lane-ops/s", "peak": lane_peak, "peak_source": f"{sms} SMs x 128 lanes x {mhz:.0f} MHz"}
     if splat_ms:
         ops = 9 * pairs
-        comp["k_splat"] = {"pairs": pairs, "pairs_per_s": pairs / (splat_ms / 1000), "ops_per_pair": 9,
+        comp["surface_bake"] = {"pairs": pairs, "pairs_per_s": pairs / (splat_ms / 1000), "ops_per_pair": 9,
                            "frac": ops / (splat_ms / 1000) / lane_peak}
     body_ms = prof.get("body_splat", (None, 0))[0]
     if body_ms and body_pairs:
