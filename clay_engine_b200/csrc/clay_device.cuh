@@ -1239,7 +1239,8 @@ __device__ __forceinline__ void new_velocity(const SceneDev& S, const ParamsDev&
 }
 
 // Whether cell-ordered particle k is among its own neighbours (the density pass lists it at r = 0): not outside the
-// grid, and not past the bucket of an overfull cell.
+// grid, and not past the bucket of an overfull cell. For live particles alone: their cells lie in the box of occupied
+// cells, any other position's may not, and its index into the cell table is then out of range.
 __device__ __forceinline__ bool self_listed(const SceneDev& S, const BoxInfo& b, bool overflow, uint32_t k, int cx, int cy, int cz) {
   if (cx < 0 || cy < 0 || cz < 0 || cx >= S.G || cy >= S.G || cz >= S.G) return false;
   if (!overflow) return true;
@@ -1568,7 +1569,7 @@ __global__ void __launch_bounds__(kTeamBlock) k_forces_team(const SceneDev* __re
   cell_of(S, me.x, me.y, me.z, cx, cy, cz);
   const uint32_t cnt = valid ? __float_as_uint(mdp.w) : 0u;
   float fx = 0.0f, fy = 0.0f, fz = 0.0f, vsx = 0.0f, vsy = 0.0f, vsz = 0.0f, wsum = 0.0f;
-  if (cnt > kMaxNbr || !self_listed(S, b, overflow, k, cx, cy, cz)) {
+  if (cnt > kMaxNbr || (valid && !self_listed(S, b, overflow, k, cx, cy, cz))) {
     vsx = mv.x * S.h6;
     vsy = mv.y * S.h6;
     vsz = mv.z * S.h6;

@@ -131,3 +131,47 @@ def test_upload_between_batched_frames(root, use_graph):
     b.destroy()
     for s in alone + batch_sims:
         s.destroy()
+
+
+# (particles, spacing, bucket, centre, collider, far): centres beyond the world origin on one axis and on all of them (its cell
+# is then outside the box of occupied cells), counts that fill the team passes' blocks of 32 and that do not, up to the most that
+# take them; spacing 0.07: more neighbours than a list holds; bucket 6: overfull cells; far: particles outside the grid
+CROWDS = [(1000, 0.04, 64, (0.0, 1.0, 5.0), False, 0), (1000, 0.07, 6, (5.0, 6.0, 7.0), True, 7), (1024, 0.07, 6, (5.0, 6.0, 7.0), False, 0),
+          (33, 0.05, 6, (9.0, 9.0, 9.0), False, 1), (3001, 0.07, 64, (0.5, -0.5, 0.5), True, 31), (4000, 0.07, 6, (-7.0, -1.0, -7.0), True, 0),
+          (20479, 0.07, 64, (4.0, 3.0, 4.0), True, 97), (20480, 0.09, 6, (4.0, 3.0, 4.0), False, 97)]
+
+
+@pytest.mark.parametrize("n,spacing,bucket,centre,collide,far", CROWDS)
+def test_crowded_scene_in_a_batch_equals_alone(root, n, spacing, bucket, centre, collide, far):
+    """Fast mode: a scene by itself (eight lanes a particle) and in a batch (a thread each) come out the same bits where
+    particles have more neighbours than their list holds, are past an overfull cell's bucket or outside the grid."""
+    import clay_engine_b200 as ce
+    from clay_engine_b200 import scenes
+
+    field = None
+    if collide:
+        vol = ce.SdfVolume(root, resolution=64, worldSize=24.0, origin=ORIGIN)
+        vol.build(scenes.config1_collider_brushes())
+        field = ce.volumeField(vol)
+    p = scenes.lattice_block(n, spacing, centre, n)
+    p["vel"] = np.random.default_rng(n).normal(0, 0.5, (n, 3))
+    if far:
+        p["pos"][:: n // far, 1] += 40.0
+    sims = []
+    for _ in range(2):
+        s = ce.FluidSim(root, field, dict(capacity=n + 5, spacing=0.1, radius=0.05, substeps=2, bucket=bucket, bakeResolution=16,
+                                          bakeMipLevels=1, worldSize=24.0, origin=ORIGIN))
+        s.set_mode("fast")
+        s.upload(p)
+        sims.append(s)
+    b = ce.Batch(root, [sims[0]])
+    for frame in range(3):
+        b.step()
+        sims[1].step()
+        together, alone = sims[0].download(), sims[1].download()
+        for name in ("pos", "vel", "density", "pressure", "nvel"):
+            x, y = (np.ascontiguousarray(a[name]).view(np.uint32) for a in (together, alone))
+            assert np.array_equal(x, y), f"frame {frame}: {name} of {(x != y).reshape(n, -1).any(1).sum()} particles differs"
+    b.destroy()
+    for s in sims:
+        s.destroy()
