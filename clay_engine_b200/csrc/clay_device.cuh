@@ -192,6 +192,11 @@ constexpr uint32_t kSplatTileRatio = 6, kSplatWalkWeight = 3;
 // The box tree over a cloud in spatially coherent order: 32 particles per leaf, 32 leaves per
 // group, 32 groups per super-group, each box as two float4 (low, high corner).
 constexpr uint32_t kLeafN = 32, kGroupN = 32 * kLeafN, kSuperN = 32 * kGroupN;
+// Super-groups of `n` particles (at most 2^26). Compared with a number of one, never multiplied out: a surface has up to
+// 153 M chunks (4096^3 and its levels), and from the 131,072nd on (512^3) a chunk's number times kSuperN wraps.
+__host__ __device__ constexpr uint32_t bake_supers(uint32_t n) { return (n + kSuperN - 1) / kSuperN; }
+static_assert(bake_supers(1) == 1 && bake_supers(kSuperN) == 1 && bake_supers(kSuperN + 1) == 2);
+static_assert(bake_supers(1u << 26) == 2048 && 131072u >= bake_supers(1u << 26));  // such a chunk writes none
 // Scratch of the tree of `n` particles, in 16-byte units, and where its parts start.
 struct BakeTreeLayout {
   uint64_t leaf, group, super, cursor, list, total;
@@ -2803,7 +2808,7 @@ __global__ void __launch_bounds__(32 * kMarkWarps) k_bake_mark(const SplatDev* _
     all += q * q * q;
   }
   // super-group boxes for the gather pass, spread over the object's warps
-  for (uint32_t s = c; s * kSuperN < n; s += all) {
+  for (uint32_t s = c, ns = bake_supers(n); s < ns; s += all) {
     const uint32_t g = 32u * s + lane;
     const float inf = __int_as_float(0x7f800000);
     const float4 glo = g < ng ? D.group[2 * g] : make_float4(inf, inf, inf, 0.0f);
@@ -2933,7 +2938,7 @@ struct BakeTree {
   __device__ __forceinline__ void descend(float x0, float y0, float z0, float x1, float y1, float z1, const uint32_t& best,
                                           W&& wants, F&& visit) const {
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t nl = (n + kLeafN - 1) / kLeafN, ng = (n + kGroupN - 1) / kGroupN, ns = (n + kSuperN - 1) / kSuperN;
+    const uint32_t nl = (n + kLeafN - 1) / kLeafN, ng = (n + kGroupN - 1) / kGroupN, ns = bake_supers(n);
     auto groups = [&](uint32_t s) {
       each_nearest(box_bits(group, 32 * s + lane, ng, x0, y0, z0, x1, y1, z1), best, [&](uint32_t g) {
         if (!wants(group, 32 * s + g)) return;

@@ -31,11 +31,11 @@ SCENES = [("pile", 130000, 131071, 64, 3), ("pile", 40000, 40000, 64, 2), ("pile
           ("spray", 4100, 20000, 32, 2), ("spray", 60000, 70000, 32, 1), ("spray", 3000, 3000, 64, 3), ("pile", 0, 5000, 32, 2)]
 
 
-def make(root, mode):
+def make(root, mode, wanted=SCENES):
     import clay_engine_b200 as ce
 
     sims = []
-    for i, (kind, live, cap, res, mips) in enumerate(SCENES):
+    for i, (kind, live, cap, res, mips) in enumerate(wanted):
         s = ce.FluidSim(root, None, dict(capacity=cap, spacing=0.1, radius=0.05, substeps=2, bakeResolution=res,
                                          bakeMipLevels=mips, bakeBand=(2.0, 4.0, 3.0)[i % 3], worldSize=24.0, origin=ORIGIN))
         s.set_mode(mode)
@@ -71,5 +71,24 @@ def test_gathered_batch_equals_splatted_scenes(root, lanes):
         gd, ad = x.surface.volume.download()[0], y.surface.volume.download()[0]
         assert np.array_equal(gd, ad), f"scene {i} {SCENES[i]}: {(gd != ad).sum()} voxels differ"
         assert (ad != 0x3C00).any() == (SCENES[i][1] > 0)
+    for o in [b] + together + alone:
+        o.destroy()
+
+
+def test_gathered_surface_of_many_chunks_equals_splatted(root):
+    """A small dense scene with a surface of more than 131,072 chunks of 8^3 voxels: its super-groups are counted, and a
+    chunk's number times their 32,768 particles (which passes 2^32 there) decides nothing."""
+    import clay_engine_b200 as ce
+
+    wanted = [("pile", 8192, 8200, 416, 2), ("pile", 40000, 255000, 64, 2)]
+    assert (416 // 8) ** 3 + (208 // 8) ** 3 > 1 << 17 and sum(c for _, _, c, _, _ in wanted) >= 1 << 18
+    together, alone = make(root, "reference", wanted), make(root, "reference", wanted)
+    b = ce.Batch(root, together)
+    b.step()
+    for i, (x, y) in enumerate(zip(together, alone)):
+        y.step()
+        gd, ad = x.surface.volume.download()[0], y.surface.volume.download()[0]
+        assert np.array_equal(gd, ad), f"scene {i}: {(gd != ad).sum()} voxels differ"
+        assert (ad != 0x3C00).any()
     for o in [b] + together + alone:
         o.destroy()
