@@ -229,6 +229,44 @@ struct clay_field {
   }
 };
 
+// A branch beside a stream's work: what runs on it starts after the work before it on that stream and is waited for by
+// what follows join. Works under stream capture too.
+struct Branch {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t fork = nullptr, done = nullptr;
+  Branch() = default;
+  Branch(const Branch&) = delete;
+  Branch(Branch&& o) noexcept : stream(o.stream), fork(o.fork), done(o.done) {
+    o.stream = nullptr;
+    o.fork = o.done = nullptr;
+  }
+  Branch& operator=(const Branch&) = delete;
+  ~Branch() {
+    if (stream) cudaStreamDestroy(stream);
+    if (fork) cudaEventDestroy(fork);
+    if (done) cudaEventDestroy(done);
+  }
+  int create() {
+    if (!stream) CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+    if (!fork) CK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+    if (!done) CK(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
+    return CLAY_OK;
+  }
+  int begin(cudaStream_t s) {
+    CK(cudaEventRecord(fork, s));
+    CK(cudaStreamWaitEvent(stream, fork, 0));
+    return CLAY_OK;
+  }
+  int end() {
+    CK(cudaEventRecord(done, stream));
+    return CLAY_OK;
+  }
+  int join(cudaStream_t s) {
+    CK(cudaStreamWaitEvent(s, done, 0));
+    return CLAY_OK;
+  }
+};
+
 struct clay_splat {
   clay_ctx* ctx = nullptr;
   clay_volume* vol = nullptr;
@@ -239,22 +277,23 @@ struct clay_splat {
   uint32_t* keys = nullptr;
   SplatDev h{};
   SplatDev* d = nullptr;          // cloud in index order
-  // fluid-owned splats: the fluid's cloud in cell order, as the splat (d_plain) and the gather see it
-  SplatDev *d_plain = nullptr, *d_ordered = nullptr;
+  SplatDev* d_ordered = nullptr;  // the fluid's cloud in cell order (fluid-owned splats)
   const uint32_t* order = nullptr;
   // A fluid's surface may be baked by gathering over a box tree of the cell-ordered cloud, in
   // scratch that the fluid's neighbour lists leave free once the last substep has read them.
   float4* tree = nullptr;
   bool sorted = false;  // gathered in Morton order
   const GridState* gs = nullptr;
+  Branch branch;  // the gather's launches beside the splat's, of a scene by itself
   bool desc_dirty = true;
 
   // Blocks of 8 x 4 x 2 voxels over all levels: the most a bake's list holds.
   int64_t blocks() const { return vol->total / 64; }
-  // `gather`: the device chooses how to bake it, else it is splatted.
-  void bind_tree(SplatDev* o, bool gather) const {
+  // Whether the device may gather it at all.
+  bool gatherable() const { return gs && cloud.capacity >= kGatherMin; }
+  void bind_tree(SplatDev* o) const {
     o->order = order;
-    if (!gather || cloud.capacity < kGatherMin) return;
+    if (!gatherable()) return;
     const BakeTreeLayout l = bake_tree_layout(cloud.capacity);
     o->gs = gs;
     o->bpos = tree;
@@ -263,10 +302,8 @@ struct clay_splat {
     o->super = tree + l.super;
     o->cursor = sorted ? reinterpret_cast<uint32_t*>(tree + l.cursor) : nullptr;
   }
-  // Whether `live` particles baked by themselves are gathered (bake_gathers' second rule, which they then fulfil).
-  bool gathers(int64_t live) const {
-    return gs && live >= kGatherAlone && 8 * live >= static_cast<int64_t>(res) * res * res && list(blocks()).items;
-  }
+  // Whether the device may gather `live` particles baked by themselves.
+  bool may_gather(int64_t live) const { return branch.stream && live >= kGatherAlone && list(blocks()).items; }
   // A bake list of `items` blocks in what the tree leaves of the neighbour lists' memory (NULL where it does not fit).
   BakeList list(int64_t items) const {
     const uint64_t at = bake_tree_layout(cloud.capacity).list, slots = static_cast<uint64_t>(cloud.capacity) * (kMaxNbr / 4);
@@ -288,10 +325,7 @@ struct clay_splat {
     if (rc) return rc;
     if (d_ordered) {
       SplatDev o = h;
-      bind_tree(&o, false);
-      rc = ctx->upload(d_plain, &o, sizeof(o), s);
-      if (rc) return rc;
-      bind_tree(&o, true);
+      bind_tree(&o);
       rc = ctx->upload(d_ordered, &o, sizeof(o), s);
       if (rc) return rc;
     }
@@ -519,9 +553,8 @@ int make_splat(clay_ctx* ctx, const clay_cloud_desc* cloud, const clay_splat_opt
   if ((rc = ctx->dev_alloc(&p, sizeof(SplatDev)))) goto fail_out;
   s->d = static_cast<SplatDev*>(p);
   if (with_order) {
-    if ((rc = ctx->dev_alloc(&p, 2 * sizeof(SplatDev)))) goto fail_out;
-    s->d_plain = static_cast<SplatDev*>(p);
-    s->d_ordered = s->d_plain + 1;
+    if ((rc = ctx->dev_alloc(&p, sizeof(SplatDev)))) goto fail_out;
+    s->d_ordered = static_cast<SplatDev*>(p);
   }
   {
     SplatDev& h = s->h;
@@ -566,7 +599,7 @@ int make_splat(clay_ctx* ctx, const clay_cloud_desc* cloud, const clay_splat_opt
 fail_out:
   if (s->keys) ctx->dev_free(s->keys, sizeof(uint32_t) * vol->total);
   if (s->d) ctx->dev_free(s->d, sizeof(SplatDev));
-  if (s->d_plain) ctx->dev_free(s->d_plain, 2 * sizeof(SplatDev));
+  if (s->d_ordered) ctx->dev_free(s->d_ordered, sizeof(SplatDev));
   free_field(s->field);
   free_volume(vol);
   delete s;
@@ -577,7 +610,7 @@ void free_splat(clay_splat* s) {
   if (!s) return;
   s->ctx->dev_free(s->keys, sizeof(uint32_t) * s->vol->total);
   s->ctx->dev_free(s->d, sizeof(SplatDev));
-  if (s->d_plain) s->ctx->dev_free(s->d_plain, 2 * sizeof(SplatDev));
+  if (s->d_ordered) s->ctx->dev_free(s->d_ordered, sizeof(SplatDev));
   free_field(s->field);
   free_volume(s->vol);
   delete s;
@@ -595,35 +628,39 @@ int64_t discs_per_block(Blocks&& blocks) {
 }
 
 // Blocks over the cloud's iteration space for every mip (plain bake), of a fluid (`scene`) in cell
-// order; a large fluid is gathered.
+// order. A large fluid's splat and gather are both launched and the device takes one of them; the launches of the
+// other, some 4 us each by themselves (a frame of 262,144 particles 268 -> 292 us), pass beside it.
 int splat_bake(clay_splat* s, cudaStream_t st, const SceneDev* scene, int64_t iter_n) {
   int rc = s->flush(st);
   if (rc) return rc;
   int64_t n = iter_n;
-  if (scene && s->gathers(n)) {
+  const bool choose = scene && s->may_gather(n);
+  if (choose) {
     const BakeList list = s->list(s->blocks());
+    if ((rc = s->branch.begin(st))) return rc;
+    const cudaStream_t bs = s->branch.stream;
     if (s->sorted) {
-      CK(L_sort_scan(scene, s->d_ordered, nullptr, s->sort_parts(), false, st));
-      CK(L_sort_scan(scene, s->d_ordered, nullptr, s->sort_parts(), true, st));
-      CK(L_sort_scatter(scene, s->d_ordered, nullptr, static_cast<int>((n + 255) / 256), st));
+      CK(L_sort_scan(scene, s->d_ordered, nullptr, s->sort_parts(), false, bs));
+      CK(L_sort_scan(scene, s->d_ordered, nullptr, s->sort_parts(), true, bs));
+      CK(L_sort_scatter(scene, s->d_ordered, nullptr, static_cast<int>((n + 255) / 256), bs));
     }
-    CK(L_bake_tree(s->d_ordered, nullptr, static_cast<int>((n + kGroupN - 1) / kGroupN), list, st));
-    CK(L_bake_mark(s->d_ordered, nullptr, mark_blocks(s), list, st));
-    CK(L_bake_gather(s->d_ordered, static_cast<int>(std::min<int64_t>(kGatherBlocks, s->blocks())), list, st));
-    return CLAY_OK;
+    CK(L_bake_tree(s->d_ordered, nullptr, static_cast<int>((n + kGroupN - 1) / kGroupN), list, bs));
+    CK(L_bake_mark(s->d_ordered, nullptr, mark_blocks(s), list, bs));
+    CK(L_bake_gather(s->d_ordered, static_cast<int>(std::min<int64_t>(kGatherBlocks, s->blocks())), list, bs));
+    if ((rc = s->branch.end())) return rc;
   }
-  const SplatDev* d = scene ? s->d_plain : s->d;
+  const SplatDev* d = scene ? s->d_ordered : s->d;
   if (n > 0) {
     // a small disc cloud in blocks of fewer particles, until they fill the device (see k_splat)
     const int64_t per = s->cloud.normals ? discs_per_block([&](int64_t p) { return (n + p - 1) / p * s->mips; }) : kSplatThreads;
     int blocks = static_cast<int>((n + per - 1) / per);
-    CK(L_splat(d, nullptr, blocks, s->mips, s->cloud.normals ? kSplatAccVoxelsDiscs : kSplatAccVoxels, st,
+    CK(L_splat(d, nullptr, blocks, s->mips, s->cloud.normals ? kSplatAccVoxelsDiscs : kSplatAccVoxels, choose, st,
                static_cast<uint32_t>(per)));
   }
   int64_t quads = (s->vol->total + 3) / 4;
   int rblocks = static_cast<int>((quads + kResolveThreads - 1) / kResolveThreads);
-  CK(L_resolve(d, nullptr, rblocks, st));
-  return CLAY_OK;
+  CK(L_resolve(d, nullptr, rblocks, choose, st));
+  return choose ? s->branch.join(st) : CLAY_OK;
 }
 
 }  // namespace
@@ -1044,7 +1081,7 @@ int clay_fluid_estimate_bytes(const clay_fluid_opts* opts, uint64_t* out) {
     t += r * r * r;
   }
   // volume planes (f16 distance, f16 material) and uniform, its field, the key grid, descriptors
-  b += t * (2 * sizeof(__half) + sizeof(uint32_t)) + sizeof(VolParamsDev) + sizeof(FieldDev) + 3 * sizeof(SplatDev);
+  b += t * (2 * sizeof(__half) + sizeof(uint32_t)) + sizeof(VolParamsDev) + sizeof(FieldDev) + 2 * sizeof(SplatDev);
   *out = b;
   return CLAY_OK;
 }
@@ -1157,6 +1194,7 @@ int clay_fluid_create(clay_ctx* ctx, const clay_field* world, const clay_fluid_o
   f->surface->gs = f->substeps > 0 ? f->gs : nullptr;  // without substeps there is no cell order
   f->surface->desc_dirty = true;
   rc = f->surface->flush(nullptr);
+  if (!rc && f->surface->gatherable() && C >= kGatherAlone) rc = f->surface->branch.create();
   if (rc) {
     clay_fluid_destroy(f);
     return rc;
@@ -1448,15 +1486,15 @@ struct clay_batch {
   size_t n_scenes_alloc = 0;
   SplatDev* d_extra = nullptr;   // extra clouds, index order
   SplatDev* d_surf = nullptr;    // fluid surfaces, cell order
-  SplatDev* d_surf_splat = nullptr;  // the same, always splatted
   Work *w_emit = nullptr, *w_scan = nullptr, *w_xsplat = nullptr, *w_xres = nullptr,
        *w_ssplat = nullptr, *w_sres = nullptr, *w_sort = nullptr, *w_scatter = nullptr, *w_tree = nullptr, *w_mark = nullptr;
   int n_part = 0, n_emit = 0, n_scan = 0, n_xsplat = 0, n_xres = 0, n_ssplat = 0, n_sres = 0, n_sort = 0, n_scatter = 0, n_tree = 0, n_mark = 0;
   int n_gather = 0;
-  bool gather = false;  // the device chooses per scene between the splat and the gather
+  bool gather = false;  // the tables let the device choose per scene between the splat and the gather
   std::vector<DevBuf> bufs;
   bool built = false;
-  cudaGraphExec_t graph = nullptr;
+  cudaGraphExec_t graph[2] = {nullptr, nullptr};  // a frame that splats every surface, one that may gather
+  int64_t graph_launches[2] = {0, 0};
   // Per scene-size bucket thread-block size of the particle passes: a scene whose capacity is
   // below bucket_upper[i] uses bucket_block[i]; others use tune.sph_block. One launch per
   // distinct block size per pass.
@@ -1481,6 +1519,7 @@ struct clay_batch {
     Work *w_emit = nullptr, *w_scan = nullptr, *w_ssplat = nullptr, *w_sres = nullptr, *w_sort = nullptr, *w_scatter = nullptr, *w_tree = nullptr, *w_mark = nullptr;
     int n_part = 0, n_emit = 0, n_scan = 0, n_ssplat = 0, n_sres = 0, n_sort = 0, n_scatter = 0, n_tree = 0, n_mark = 0, n_gather = 0;
     BakeList list{};
+    Branch bake;                    // the gather's launches beside the splat's
     cudaStream_t stream = nullptr;  // lane 0 runs on the frame's stream
     cudaEvent_t done = nullptr;
   };
@@ -1549,9 +1588,9 @@ struct clay_batch {
     if (d_sub) ctx->dev_free(d_sub, d_sub_cap * sizeof(Work));
   }
   void release() {
-    if (graph) {
-      cudaGraphExecDestroy(graph);
-      graph = nullptr;
+    for (cudaGraphExec_t& g : graph) {
+      if (g) cudaGraphExecDestroy(g);
+      g = nullptr;
     }
     for (int k = 0; k < 2; k++) {
       if (h_params[k]) cudaFreeHost(h_params[k]);
@@ -1599,12 +1638,14 @@ struct clay_batch {
 
 namespace {
 
-void add_splat_work(std::vector<Work>& ws, std::vector<Work>& wr, uint32_t obj, const clay_splat* s, int64_t iter_n,
-                    int splat_block) {
+void add_splat_work(std::vector<Work>& ws, uint32_t obj, const clay_splat* s, int64_t iter_n, int splat_block) {
   for (int m = 0; m < s->mips; m++)
     for (int64_t f = 0; f < iter_n; f += splat_block)
       ws.push_back({obj, static_cast<uint32_t>(m), static_cast<uint32_t>(f),
                     static_cast<uint32_t>(std::min<int64_t>(splat_block, iter_n - f))});
+}
+
+void add_resolve_work(std::vector<Work>& wr, uint32_t obj, const clay_splat* s) {
   int64_t quads = (s->vol->total + 3) / 4;
   for (int64_t q = 0; q < quads; q += kResolveThreads) wr.push_back({obj, 0u, static_cast<uint32_t>(q), kResolveThreads});
 }
@@ -1630,7 +1671,7 @@ BakeList batch_list(const clay_batch* b, const Scenes& scenes) {
   int64_t items = 0;
   for (int i : scenes) {
     const clay_splat* s = b->sims[static_cast<size_t>(i)]->surface;
-    if (!s->gs || s->cloud.capacity < kGatherMin) continue;
+    if (!s->gatherable()) continue;
     items += s->blocks();
     if (!largest || s->cloud.capacity > largest->cloud.capacity) largest = s;
   }
@@ -1671,7 +1712,7 @@ int batch_build(clay_batch* b) {
     for (int e = 0; e < eb; e++) we.push_back({obj, 0u, static_cast<uint32_t>(e * T), static_cast<uint32_t>(eb * T)});
     for (uint32_t p = 0; p < f->batch_parts; p++) wsc.push_back({obj, p, 0u, 0u});
   }
-  std::vector<SplatDev> xs, ss, sp;
+  std::vector<SplatDev> xs, ss;
   std::vector<Work> wxs, wxr, wss, wsr, wso, wsc2, wtr, wmk;
   int64_t items = 0, particles = 0;
   for (const clay_fluid* f : b->sims) particles += f->capacity;
@@ -1707,19 +1748,21 @@ int batch_build(clay_batch* b) {
   for (size_t i = 0; i < b->extra.size(); i++) {
     xs.push_back(b->extra[i]->h);
     xs.back().order = nullptr;
-    add_splat_work(wxs, wxr, static_cast<uint32_t>(i), b->extra[i], b->extra[i]->cloud.capacity,
+    add_splat_work(wxs, static_cast<uint32_t>(i), b->extra[i], b->extra[i]->cloud.capacity,
                    b->extra[i]->cloud.normals ? static_cast<int>(disc_block) : kSplatThreads);
+    add_resolve_work(wxr, static_cast<uint32_t>(i), b->extra[i]);
   }
   for (size_t i = 0; i < b->sims.size(); i++) {
     clay_splat* s = b->sims[i]->surface;
     SplatDev d = s->h;
-    s->bind_tree(&d, b->gather);
+    s->bind_tree(&d);
     const clay_bucket_tuning bt = b->tuning_of(b->sims[i]->capacity);
     d.tile_ratio = static_cast<uint32_t>(bt.splat_tile_ratio);
     d.walk_weight = static_cast<uint32_t>(bt.splat_walk_weight);
     ss.push_back(d);
-    add_splat_work(wss, wsr, static_cast<uint32_t>(i), s, b->sims[i]->capacity, kSplatThreads);
-    if (!d.gs) continue;
+    add_splat_work(wss, static_cast<uint32_t>(i), s, b->sims[i]->capacity, kSplatThreads);
+    add_resolve_work(wsr, static_cast<uint32_t>(i), s);
+    if (!b->gather || !d.gs) continue;
     add_bake_work(wso, wsc2, wtr, wmk, static_cast<uint32_t>(i), s, b->sims[i]->capacity);
     items += s->blocks();
   }
@@ -1730,7 +1773,7 @@ int batch_build(clay_batch* b) {
     const size_t tables = static_cast<size_t>(nl + 1) * (blocks.size() + 12);
     const size_t bytes = (nl > 1 ? 2 : 1) * works * sizeof(Work) + tables * 256 + clay_batch::table_bytes<ParamsDev>(b->sims.size()) +
                          clay_batch::table_bytes<ContactsDev>(b->sims.size()) + clay_batch::table_bytes<SceneDev>(scenes.size()) +
-                         clay_batch::table_bytes<SplatDev>(xs.size()) + 2 * clay_batch::table_bytes<SplatDev>(ss.size());
+                         clay_batch::table_bytes<SplatDev>(xs.size()) + clay_batch::table_bytes<SplatDev>(ss.size());
     if ((rc = b->reserve_tables(bytes))) return rc;
   }
   {
@@ -1743,8 +1786,6 @@ int batch_build(clay_batch* b) {
       scenes[i].prm = b->d_params + i;
       ss[i].live_count = &b->d_params[i].count;
     }
-    sp = ss;
-    for (SplatDev& d : sp) d.gs = nullptr;
     for (int k = 0; k < 2; k++) {
       CK(cudaMallocHost(&b->h_params[k], sizeof(ParamsDev) * std::max<size_t>(b->sims.size(), 1)));
       if (!b->params_ev[k]) CK(cudaEventCreateWithFlags(&b->params_ev[k], cudaEventDisableTiming));
@@ -1752,7 +1793,7 @@ int batch_build(clay_batch* b) {
   }
   if ((rc = b->upload_table(&b->d_scenes, scenes)) ||
       (rc = b->upload_table(&b->w_emit, we)) || (rc = b->upload_table(&b->w_scan, wsc)) ||
-      (rc = b->upload_table(&b->d_extra, xs)) || (rc = b->upload_table(&b->d_surf, ss)) || (rc = b->upload_table(&b->d_surf_splat, sp)) ||
+      (rc = b->upload_table(&b->d_extra, xs)) || (rc = b->upload_table(&b->d_surf, ss)) ||
       (rc = b->upload_table(&b->w_xsplat, wxs)) || (rc = b->upload_table(&b->w_xres, wxr)) ||
       (rc = b->upload_table(&b->w_sort, wso)) || (rc = b->upload_table(&b->w_scatter, wsc2)) ||
       (rc = b->upload_table(&b->w_ssplat, wss)) || (rc = b->upload_table(&b->w_sres, wsr)) ||
@@ -1773,7 +1814,6 @@ int batch_build(clay_batch* b) {
       if (b->lanes[l].done) cudaEventDestroy(b->lanes[l].done);
     }
     b->lanes.resize(static_cast<size_t>(nl));
-    for (size_t l = old_lanes; l < b->lanes.size(); l++) b->lanes[l] = clay_batch::Lane{};
     for (int l = 0; l < nl; l++) {
       clay_batch::Lane& ln = b->lanes[static_cast<size_t>(l)];
       auto mine = [&](const std::vector<Work>& all) {
@@ -1782,6 +1822,7 @@ int batch_build(clay_batch* b) {
           if (lane_of[w.obj] == l) out.push_back(w);
         return out;
       };
+      if (b->gather && (rc = ln.bake.create())) return rc;
       ln.groups.clear();
       ln.n_part = 0;
       if (nl == 1) {  // one lane: every scene, in the batch's own tables
@@ -1850,10 +1891,21 @@ int batch_build(clay_batch* b) {
   return CLAY_OK;
 }
 
+// Whether a frame of the batch may gather surfaces: its scenes hold enough particles now. A capacity that
+// is not filled yet costs the gather's launches for nothing (12 scenes of 2,000 in 65,536 places: 244 us a frame
+// without them, 266 with).
+bool batch_gathers(const clay_batch* b) {
+  int64_t live = 0;
+  for (const clay_fluid* f : b->sims) live += f->live;
+  return b->gather && live >= kGatherBatch;
+}
+
 // The passes of one batched frame. Order as in a game frame: the extra clouds (clay-body
 // shells, which the fluids collide with) bake first, then every fluid steps and bakes.
-int batch_enqueue(clay_batch* b, cudaStream_t s) {
+// `gather`: the device may gather surfaces (see batch_gathers).
+int batch_enqueue(clay_batch* b, bool gather, cudaStream_t s) {
   const int T = b->tune.sph_block;
+  const SplatDev* surf = b->d_surf;
   const SceneDev* d = b->d_scenes;
   const bool multi = b->lanes.size() > 1;
   // the extra clouds' bake: on the side stream when there are fluids to overlap it with
@@ -1861,12 +1913,12 @@ int batch_enqueue(clay_batch* b, cudaStream_t s) {
   if (fork || multi) CK(cudaEventRecord(b->ev_fork, s));  // the stream and events exist from batch_build on
   if (fork) {
     CK(cudaStreamWaitEvent(b->side, b->ev_fork, 0));
-    CK(L_splat(b->d_extra, b->w_xsplat, b->n_xsplat, 1, kSplatAccVoxelsDiscs, b->side));
-    if (b->n_xres) CK(L_resolve(b->d_extra, b->w_xres, b->n_xres, b->side));
+    CK(L_splat(b->d_extra, b->w_xsplat, b->n_xsplat, 1, kSplatAccVoxelsDiscs, false, b->side));
+    if (b->n_xres) CK(L_resolve(b->d_extra, b->w_xres, b->n_xres, false, b->side));
     CK(cudaEventRecord(b->ev_join, b->side));
   } else {
-    if (b->n_xsplat) CK(L_splat(b->d_extra, b->w_xsplat, b->n_xsplat, 1, kSplatAccVoxelsDiscs, s));
-    if (b->n_xres) CK(L_resolve(b->d_extra, b->w_xres, b->n_xres, s));
+    if (b->n_xsplat) CK(L_splat(b->d_extra, b->w_xsplat, b->n_xsplat, 1, kSplatAccVoxelsDiscs, false, s));
+    if (b->n_xres) CK(L_resolve(b->d_extra, b->w_xres, b->n_xres, false, s));
   }
   for (size_t li = 0; li < b->lanes.size(); li++) {
     clay_batch::Lane& ln = b->lanes[li];
@@ -1897,17 +1949,26 @@ int batch_enqueue(clay_batch* b, cudaStream_t s) {
       }
     }
     if (!joined) CK(cudaStreamWaitEvent(ls, b->ev_join, 0));
-    if (ln.n_ssplat) CK(L_splat(b->d_surf, ln.w_ssplat, ln.n_ssplat, 1, kSplatAccVoxels, ls));
-    if (ln.n_sres) CK(L_resolve(b->d_surf, ln.w_sres, ln.n_sres, ls));
-    if (ln.n_sort) {
-      CK(L_sort_scan(d, b->d_surf, ln.w_sort, ln.n_sort, false, ls));
-      CK(L_sort_scan(d, b->d_surf, ln.w_sort, ln.n_sort, true, ls));
-      CK(L_sort_scatter(d, b->d_surf, ln.w_scatter, ln.n_scatter, ls));
+    const bool branch = gather && ln.n_tree;
+    if (branch) {
+      int rc = ln.bake.begin(ls);
+      if (rc) return rc;
+      const cudaStream_t bs = ln.bake.stream;
+      if (ln.n_sort) {
+        CK(L_sort_scan(d, surf, ln.w_sort, ln.n_sort, false, bs));
+        CK(L_sort_scan(d, surf, ln.w_sort, ln.n_sort, true, bs));
+        CK(L_sort_scatter(d, surf, ln.w_scatter, ln.n_scatter, bs));
+      }
+      CK(L_bake_tree(surf, ln.w_tree, ln.n_tree, ln.list, bs));
+      CK(L_bake_mark(surf, ln.w_mark, ln.n_mark, ln.list, bs));
+      CK(L_bake_gather(surf, ln.n_gather, ln.list, bs));
+      if ((rc = ln.bake.end())) return rc;
     }
-    if (ln.n_tree) {
-      CK(L_bake_tree(b->d_surf, ln.w_tree, ln.n_tree, ln.list, ls));
-      CK(L_bake_mark(b->d_surf, ln.w_mark, ln.n_mark, ln.list, ls));
-      CK(L_bake_gather(b->d_surf, ln.n_gather, ln.list, ls));
+    if (ln.n_ssplat) CK(L_splat(surf, ln.w_ssplat, ln.n_ssplat, 1, kSplatAccVoxels, gather, ls));
+    if (ln.n_sres) CK(L_resolve(surf, ln.w_sres, ln.n_sres, gather, ls));
+    if (branch) {
+      const int rc = ln.bake.join(ls);
+      if (rc) return rc;
     }
     if (li > 0) CK(cudaEventRecord(ln.done, ls));
   }
@@ -2034,30 +2095,33 @@ int clay_batch_step(clay_batch* b, void* stream) {
     if ((rc = x->flush(s))) return rc;
   for (clay_fluid* f : b->sims)
     if ((rc = f->surface->flush(s))) return rc;
+  const bool gather = batch_gathers(b);
   if (!b->tune.use_graph) {
     uint64_t before = launch_count();
-    rc = batch_enqueue(b, s);
+    rc = batch_enqueue(b, gather, s);
     b->launches_per_step = static_cast<int64_t>(launch_count() - before);
     return rc;
   }
-  if (!b->graph) {
+  cudaGraphExec_t& graph = b->graph[gather];
+  if (!graph) {
     // Capture on a private stream so the caller's stream can be the legacy default.
     cudaStream_t cs;
     CK(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
     cudaGraph_t g;
     CK(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
     uint64_t before = launch_count();
-    rc = batch_enqueue(b, cs);
-    b->launches_per_step = static_cast<int64_t>(launch_count() - before);
+    rc = batch_enqueue(b, gather, cs);
+    b->graph_launches[gather] = static_cast<int64_t>(launch_count() - before);
     cudaError_t e = cudaStreamEndCapture(cs, &g);
     cudaStreamDestroy(cs);
     if (rc) return rc;
     if (e != cudaSuccess) return fail(CLAY_ECUDA, "cudaStreamEndCapture: %s", cudaGetErrorString(e));
-    e = cudaGraphInstantiate(&b->graph, g, 0);
+    e = cudaGraphInstantiate(&graph, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return fail(CLAY_ECUDA, "cudaGraphInstantiate: %s", cudaGetErrorString(e));
   }
-  CK(cudaGraphLaunch(b->graph, s));
+  CK(cudaGraphLaunch(graph, s));
+  b->launches_per_step = b->graph_launches[gather];
   count_launches(static_cast<uint64_t>(b->launches_per_step));
   return CLAY_OK;
 }
@@ -2118,8 +2182,8 @@ int clay_batch_profile(clay_batch* b, void* stream, clay_phase_time* out, int ca
   const int T = b->tune.sph_block;
   const SceneDev* d = b->d_scenes;
   const bool ref = b->mode == CLAY_MODE_REFERENCE;
-  if (b->n_xsplat && (rc = timed("body_splat", [&] { return L_splat(b->d_extra, b->w_xsplat, b->n_xsplat, 1, kSplatAccVoxelsDiscs, s); }))) return rc;
-  if (b->n_xres && (rc = timed("body_resolve", [&] { return L_resolve(b->d_extra, b->w_xres, b->n_xres, s); }))) return rc;
+  if (b->n_xsplat && (rc = timed("body_splat", [&] { return L_splat(b->d_extra, b->w_xsplat, b->n_xsplat, 1, kSplatAccVoxelsDiscs, false, s); }))) return rc;
+  if (b->n_xres && (rc = timed("body_resolve", [&] { return L_resolve(b->d_extra, b->w_xres, b->n_xres, false, s); }))) return rc;
   if (b->n_part) {
     if ((rc = timed("emit", [&] { return L_emit(d, b->w_emit, b->n_emit, T, s); }))) return rc;
     for (int sub = 0; sub < b->max_substeps; sub++) {
@@ -2147,20 +2211,22 @@ int clay_batch_profile(clay_batch* b, void* stream, clay_phase_time* out, int ca
           return rc;
     }
   }
-  if (b->n_ssplat && (rc = timed("splat", [&] { return L_splat(b->d_surf, b->w_ssplat, b->n_ssplat, 1, kSplatAccVoxels, s); }))) return rc;
-  if (b->n_sres && (rc = timed("resolve", [&] { return L_resolve(b->d_surf, b->w_sres, b->n_sres, s); }))) return rc;
-  if (b->n_sort) {
-    if ((rc = timed("bake_sort", [&] { return L_sort_scan(d, b->d_surf, b->w_sort, b->n_sort, false, s); }))) return rc;
-    if ((rc = timed("bake_sort", [&] { return L_sort_scan(d, b->d_surf, b->w_sort, b->n_sort, true, s); }))) return rc;
-    if ((rc = timed("bake_scatter", [&] { return L_sort_scatter(d, b->d_surf, b->w_scatter, b->n_scatter, s); }))) return rc;
+  const bool gather = batch_gathers(b);
+  const SplatDev* surf = b->d_surf;
+  if (b->n_ssplat && (rc = timed("splat", [&] { return L_splat(surf, b->w_ssplat, b->n_ssplat, 1, kSplatAccVoxels, gather, s); }))) return rc;
+  if (b->n_sres && (rc = timed("resolve", [&] { return L_resolve(surf, b->w_sres, b->n_sres, gather, s); }))) return rc;
+  if (gather && b->n_sort) {
+    if ((rc = timed("bake_sort", [&] { return L_sort_scan(d, surf, b->w_sort, b->n_sort, false, s); }))) return rc;
+    if ((rc = timed("bake_sort", [&] { return L_sort_scan(d, surf, b->w_sort, b->n_sort, true, s); }))) return rc;
+    if ((rc = timed("bake_scatter", [&] { return L_sort_scatter(d, surf, b->w_scatter, b->n_scatter, s); }))) return rc;
   }
-  if (b->n_tree) {
+  if (gather && b->n_tree) {
     std::vector<int> all(b->sims.size());
     for (size_t i = 0; i < all.size(); i++) all[i] = static_cast<int>(i);
     const BakeList list = batch_list(b, all);
-    if ((rc = timed("bake_tree", [&] { return L_bake_tree(b->d_surf, b->w_tree, b->n_tree, list, s); }))) return rc;
-    if ((rc = timed("bake_mark", [&] { return L_bake_mark(b->d_surf, b->w_mark, b->n_mark, list, s); }))) return rc;
-    if ((rc = timed("bake_gather", [&] { return L_bake_gather(b->d_surf, b->n_gather, list, s); }))) return rc;
+    if ((rc = timed("bake_tree", [&] { return L_bake_tree(surf, b->w_tree, b->n_tree, list, s); }))) return rc;
+    if ((rc = timed("bake_mark", [&] { return L_bake_mark(surf, b->w_mark, b->n_mark, list, s); }))) return rc;
+    if ((rc = timed("bake_gather", [&] { return L_bake_gather(surf, b->n_gather, list, s); }))) return rc;
   }
   CK(cudaStreamSynchronize(s));
   std::vector<clay_phase_time> agg;
@@ -2256,19 +2322,26 @@ int clay_batch_step_subset(clay_batch* b, const int32_t* scenes, int n, void* st
     for (uint32_t p = 0; p < f->batch_parts; p++) tab.push_back({static_cast<uint32_t>(scenes[q]), p, 0u, 0u});
   }
   const int n_scan = mark() - o_scan;
-  // the splat's tables, and the gather's for the scenes that the device may gather
-  std::vector<Work> splat, resolve, sort, scatter, tree, marks;
+  auto baked = [&](int i) { return b->sims[i]->substeps > 0 ? b->sims[i]->live : 0; };
+  const int o_splat = mark();
+  for (int q = 0; q < n; q++)
+    add_splat_work(tab, static_cast<uint32_t>(scenes[q]), b->sims[scenes[q]]->surface, baked(scenes[q]), kSplatThreads);
+  const int n_splat = mark() - o_splat;
+  const int o_res = mark();
+  for (int q = 0; q < n; q++) add_resolve_work(tab, static_cast<uint32_t>(scenes[q]), b->sims[scenes[q]]->surface);
+  const int n_res = mark() - o_res;
+  // the gather's tables, for the scenes that the device may gather
   int64_t items = 0, particles = 0;
   for (int q = 0; q < n; q++) particles += b->sims[scenes[q]]->live;
-  const BakeList list = batch_list(b, std::vector<int>(scenes, scenes + n));
-  const bool gather = b->gather && particles >= kGatherBatch && list.items;
-  for (int q = 0; q < n; q++) {
-    clay_fluid* f = b->sims[scenes[q]];
-    const int64_t it = (f->substeps > 0 && f->live > 0) ? f->live : 0;
-    add_splat_work(splat, resolve, static_cast<uint32_t>(scenes[q]), f->surface, it, kSplatThreads);
-    if (!gather || it < kGatherMin) continue;
-    add_bake_work(sort, scatter, tree, marks, static_cast<uint32_t>(scenes[q]), f->surface, it);
-    items += f->surface->blocks();
+  BakeList list{};
+  if (b->gather && particles >= kGatherBatch) list = batch_list(b, std::vector<int>(scenes, scenes + n));
+  const bool gather = list.items != nullptr;
+  std::vector<Work> sort, scatter, tree, marks;
+  for (int q = 0; q < n && gather; q++) {
+    const clay_splat* surface = b->sims[scenes[q]]->surface;
+    if (baked(scenes[q]) < kGatherMin) continue;
+    add_bake_work(sort, scatter, tree, marks, static_cast<uint32_t>(scenes[q]), surface, baked(scenes[q]));
+    items += surface->blocks();
   }
   auto place = [&](const std::vector<Work>& w, int& n_out) {
     const int o = mark();
@@ -2276,11 +2349,10 @@ int clay_batch_step_subset(clay_batch* b, const int32_t* scenes, int n, void* st
     tab.insert(tab.end(), w.begin(), w.end());
     return o;
   };
-  int n_splat = 0, n_res = 0, n_sort = 0, n_scatter = 0, n_tree = 0, n_mark = 0;
-  const int o_splat = place(splat, n_splat), o_res = place(resolve, n_res), o_sort = place(sort, n_sort),
-            o_scatter = place(scatter, n_scatter), o_tree = place(tree, n_tree), o_mark = place(marks, n_mark);
-  // a frame that gathers nothing takes the surfaces as plain splats
-  const SplatDev* surf = gather ? b->d_surf : b->d_surf_splat;
+  int n_sort = 0, n_scatter = 0, n_tree = 0, n_mark = 0;
+  const int o_sort = place(sort, n_sort), o_scatter = place(scatter, n_scatter), o_tree = place(tree, n_tree),
+            o_mark = place(marks, n_mark);
+  const SplatDev* surf = b->d_surf;
   // upload params + tables through double-buffered pinned memory
   int k = b->sub_slot;
   b->sub_slot ^= 1;
@@ -2329,18 +2401,23 @@ int clay_batch_step_subset(clay_batch* b, const int32_t* scenes, int n, void* st
       CK(L_forces_fast(d, W + o_part, n_part, T, sub, s));
     }
   }
-  if (n_splat) CK(L_splat(surf, W + o_splat, n_splat, 1, kSplatAccVoxels, s));
-  if (n_res) CK(L_resolve(surf, W + o_res, n_res, s));
-  if (n_sort) {
-    CK(L_sort_scan(d, surf, W + o_sort, n_sort, false, s));
-    CK(L_sort_scan(d, surf, W + o_sort, n_sort, true, s));
-    CK(L_sort_scatter(d, surf, W + o_scatter, n_scatter, s));
-  }
+  Branch& branch = b->lanes[0].bake;
   if (n_tree) {
-    CK(L_bake_tree(surf, W + o_tree, n_tree, list, s));
-    CK(L_bake_mark(surf, W + o_mark, n_mark, list, s));
-    CK(L_bake_gather(surf, static_cast<int>(std::min<int64_t>(kGatherBlocks, items)), list, s));
+    if ((rc = branch.begin(s))) return rc;
+    const cudaStream_t bs = branch.stream;
+    if (n_sort) {
+      CK(L_sort_scan(d, surf, W + o_sort, n_sort, false, bs));
+      CK(L_sort_scan(d, surf, W + o_sort, n_sort, true, bs));
+      CK(L_sort_scatter(d, surf, W + o_scatter, n_scatter, bs));
+    }
+    CK(L_bake_tree(surf, W + o_tree, n_tree, list, bs));
+    CK(L_bake_mark(surf, W + o_mark, n_mark, list, bs));
+    CK(L_bake_gather(surf, static_cast<int>(std::min<int64_t>(kGatherBlocks, items)), list, bs));
+    if ((rc = branch.end())) return rc;
   }
+  if (n_splat) CK(L_splat(surf, W + o_splat, n_splat, 1, kSplatAccVoxels, gather, s));
+  if (n_res) CK(L_resolve(surf, W + o_res, n_res, gather, s));
+  if (n_tree && (rc = branch.join(s))) return rc;
   return CLAY_OK;
 }
 

@@ -121,6 +121,8 @@ struct __align__(16) GridState {
   uint32_t L;  // bbox cells; local index L is the out-of-grid bucket
   int32_t x0, y0, z0;
   uint32_t bx, by, bz;
+  // of the last substep, counted where the scene may be gathered: cells of the box that hold a particle, particles outside the grid
+  uint32_t occupied, outside;
   uint32_t part_sum[kMaxParts];
 };
 
@@ -179,7 +181,7 @@ struct __align__(16) SplatDev {
   // most walk_weight times those of the own boxes.
   uint32_t tile_ratio, walk_weight;
   // A fluid's surface: its cell-build state, by which the device chooses between the splat and the
-  // gather (see bake_gathers). NULL: k_splat bakes the cloud, whatever it looks like.
+  // gather where a frame launches both (see bake_gathers). NULL: it is splatted.
   const GridState* gs;
   // The cloud's particles in bake order with their bounding boxes (see k_bake_tree), scratch of
   // one gather.
@@ -201,11 +203,13 @@ static_assert(bake_supers(1u << 26) == 2048 && 131072u >= bake_supers(1u << 26))
 struct BakeTreeLayout {
   uint64_t leaf, group, super, cursor, list, total;
 };
-// A cloud may be gathered from kGatherMin particles on. A scene by itself is gathered from kGatherAlone on,
-// scenes of a batch when they hold kGatherBatch together: below, the gather's launches and the latency
-// of its descents cost more than the splat (4,096 particles alone: 167 us a frame with the splat, 171 with
-// the gather; five scenes of 36,000 together: 186 and 207).
-constexpr uint32_t kGatherMin = 64, kGatherAlone = 1u << 17, kGatherBatch = 1u << 18;
+// A fluid's surface may be gathered (see bake_gathers) from kGatherMin particles on, in a scene by itself from
+// kGatherAlone, in scenes of a batch when they hold kGatherBatch together: below, the gather's launches and the latency
+// of its descents cost more than the splat. Dense scenes, splat and gather, a frame of one substep: by itself, 131,072
+// particles as a pool 161 and 171 us (32^3 x 2), as a ball 182 and 200 (64^3 x 3), 262,144 268 and 255, 309 and 284; as two
+// layers each in a batch, 100 scenes of 4,096 366 and 398 us (32^3 x 2), 8 of 32,768 245 and 275, 12 343 and 357, 64 of
+// 8,192 431 and 423.
+constexpr uint32_t kGatherMin = 8192, kGatherAlone = 1u << 18, kGatherBatch = 3u << 17;
 // Scenes of more particles than kSortMin are baked in Morton order (see k_sort_scan): at most kSortBins
 // bins, scanned in parts.
 constexpr uint32_t kSortMin = 8192, kSortBins = 1u << 18, kSortPart = 2048, kSortParts = kSortBins / kSortPart + 1;
@@ -693,6 +697,7 @@ __global__ void k_cell_key(const SceneDev* __restrict__ scenes, const Work* __re
   if (w.first == 0 && threadIdx.x == 0) {
     S.contacts->count = 0u;
     S.gs->overflow = 0u;
+    S.gs->occupied = 0u;
   }
   uint32_t lo[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu};
   uint32_t hinv[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu};
@@ -822,7 +827,7 @@ __global__ void k_scan_partial(const SceneDev* __restrict__ scenes, const Work* 
 }
 
 // Cell build, pass 3b: exclusive scan into cell_start[0 .. L+1], counts cleared behind.
-__global__ void k_scan_final(const SceneDev* __restrict__ scenes, const Work* __restrict__ work, int substep) {
+__global__ void __launch_bounds__(1024, 2) k_scan_final(const SceneDev* __restrict__ scenes, const Work* __restrict__ work, int substep) {
   Work w = get_work(work);
   const SceneDev& S = scenes[w.obj];
   if (substep >= S.substeps) return;
@@ -841,12 +846,13 @@ __global__ void k_scan_final(const SceneDev* __restrict__ scenes, const Work* __
     if (threadIdx.x == 0) s_off = o;
   }
   __syncthreads();
-  uint32_t run = s_off;
+  uint32_t run = s_off, occupied = 0;
   const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (uint32_t c0 = beg; c0 < end; c0 += 4u * blockDim.x) {
     const uint32_t c = c0 + 4u * threadIdx.x;
     const uint4 q = c < end ? scan_counts(S, c, end) : make_uint4(0u, 0u, 0u, 0u);
     const uint32_t v = (q.x + q.y) + (q.z + q.w);
+    occupied += (q.x != 0u) + (q.y != 0u) + (q.z != 0u) + (q.w != 0u);
     uint32_t x = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -883,6 +889,16 @@ __global__ void k_scan_final(const SceneDev* __restrict__ scenes, const Work* __
     run += tot;
   }
   if (end == n && threadIdx.x == 0) S.cell_start[n] = run;
+  // for bake_gathers: the occupied cells (with the particles outside the grid as one more)
+  if (substep + 1 == S.substeps && work_count(S) >= (work ? kGatherMin : kGatherAlone)) {
+    s_warp[wid] = __reduce_add_sync(0xffffffffu, occupied);
+    __syncthreads();
+    if (wid == 0) {
+      const uint32_t all = __reduce_add_sync(0xffffffffu, lane < nw ? s_warp[lane] : 0u);
+      if (lane == 0 && all) atomicAdd(&S.gs->occupied, all);
+      if (lane == 0 && end == n) S.gs->outside = run - S.cell_start[n - 1u];
+    }
+  }
 }
 
 // Cell build, pass 4: provisional placement.
@@ -1678,17 +1694,22 @@ __device__ __forceinline__ uint32_t enc_key(float sd, float bw) {
   return static_cast<uint32_t>((v + 1.0f) * 32767.5f);
 }
 
-// Whether a fluid's surface is gathered: a voxel's descent costs about as much whatever the
-// cloud, a splat's particle costs the voxels of its band (splat.ts:238-246: 300 to 400 a level), so the
-// gather wins where particles are many for the voxels that they reach. They are where the occupied box is
-// densely filled, two a cell and more (1.4 M particles in 96 piles: 0.75 -> 0.35 ms), or where there is at
-// least one for eight voxels of the finest level, however they lie (262,144 as a thin spray into
-// 128^3: 0.61 -> 0.48 ms); a spray of 113,500 into 128^3 took 0.2 ms longer. gs == NULL: always splatted.
+// Whether a fluid's surface is gathered. A splat's particle costs the voxels of its band (splat.ts:238-246: 300 to 400
+// a level), most where particles lie so far apart that each walks its own; a gather's voxel costs a descent, most where
+// boxes of 32 particles are large for the voxels. So the gather wins where the fluid fills its box: two particles a
+// cell, or, as long as there is one for eight voxels of the finest level, 1.2 a cell, or two in five cells occupied.
+// Measured over pools with a share of spray from none to nine tenths, clouds, balls, columns, layers, blobs far apart, a
+// pool with a spray up to the sky, on 32^3 to 192^3, scenes of 262,144 to 1,000,000 by themselves: 285 of 375
+// frames are gathered, 1.30 times faster on average (0.94 at worst: one layer, 119 a cell); what is left to the splat would take
+// up to 2.9 times as long by the gather (a pool of 259,000 and 2,600 in the sky, 192^3: 699 -> 2,000 us). In batches
+// of 393,216 and more 1.19 times (0.96 at worst). Particles outside the grid are in no order (one bin), and 7 % of them took a
+// cloud of 600,000 from 1,930 to 2,930 us: more than 1 in 64 are splatted.
 __device__ __forceinline__ bool bake_gathers(const SplatDev& D) {
   if (!D.gs) return false;
   const uint64_t n = min(*D.live_count, D.capacity), r = static_cast<uint64_t>(D.r[0]);
-  const uint64_t cells = D.gs->L;
-  return n >= kGatherMin && ((cells > 0 && n >= 2 * cells) || 8 * n >= r * r * r);
+  const uint64_t cells = D.gs->L, occupied = D.gs->occupied;
+  if (n < kGatherMin || cells == 0 || 64ull * D.gs->outside > n) return false;
+  return n >= 2 * cells || (8 * n >= r * r * r && (5 * n >= 6 * cells || 5 * occupied >= 2 * cells));
 }
 
 __device__ __forceinline__ bool cloud_live(const SplatDev& D, uint32_t idx, uint32_t& i) {
@@ -2533,24 +2554,25 @@ __device__ __forceinline__ void resolve_block(const SplatDev& D, const Work w) {
 }
 
 #ifndef CLAY_ONLY_NEIGHBOUR_PASSES
+// `choose`: clouds that bake_gathers takes are left to the gather.
 // `per`: particles per block where there is no work table. A small disc cloud takes fewer than 256, so that its
 // blocks fill the device: a particle's walk is a chain of its own, and a warp of a full block makes 32 of them one after
 // another (a clay body of 3,800 discs on 30 blocks: 204 us).
 __global__ void __launch_bounds__(32 * kSplatWarps, 4) k_splat(const SplatDev* __restrict__ splats, const Work* __restrict__ work,
-                                                             uint32_t acc_cap, uint32_t per) {
+                                                             uint32_t acc_cap, uint32_t per, bool choose) {
   Work w = get_work_reversed(work);
   if (!work) {
     w.first = (gridDim.x - 1u - blockIdx.x) * per;
     w.n = per;
   }
   const SplatDev& D = splats[w.obj];
-  if (bake_gathers(D)) return;
+  if (choose && bake_gathers(D)) return;
   splat_block(D, w, D.vp->origin[0], D.vp->origin[1], D.vp->origin[2], acc_cap);
 }
 
-__global__ void k_resolve(const SplatDev* __restrict__ splats, const Work* __restrict__ work) {
+__global__ void k_resolve(const SplatDev* __restrict__ splats, const Work* __restrict__ work, bool choose) {
   const Work w = get_work(work);
-  if (bake_gathers(splats[w.obj])) return;
+  if (choose && bake_gathers(splats[w.obj])) return;
   resolve_block(splats[w.obj], w);
 }
 

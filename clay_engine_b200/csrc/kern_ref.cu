@@ -64,7 +64,8 @@ cudaError_t L_forces_ref(const SceneDev* s, const Work* w, int blocks, int threa
   count_launch();
   return cudaPeekAtLastError();
 }
-cudaError_t L_splat(const SplatDev* d, const Work* w, int blocks, int blocks_y, uint32_t acc_voxels, cudaStream_t st, uint32_t per) {
+cudaError_t L_splat(const SplatDev* d, const Work* w, int blocks, int blocks_y, uint32_t acc_voxels, bool choose, cudaStream_t st,
+                    uint32_t per) {
   // The splat's shared memory exceeds the default per-block limit; the opt-in is a property
   // of the function on each device, so it is set once per device (from any thread).
   constexpr int kDevices = 64;
@@ -79,7 +80,7 @@ cudaError_t L_splat(const SplatDev* d, const Work* w, int blocks, int blocks_y, 
     if (dev >= 0 && dev < kDevices) attr_set[dev].store(true, std::memory_order_release);
   }
   dim3 g(blocks, w ? 1 : blocks_y);
-  k_splat<<<g, kSplatThreads, acc_voxels * sizeof(uint32_t), st>>>(d, w, acc_voxels, per);
+  k_splat<<<g, kSplatThreads, acc_voxels * sizeof(uint32_t), st>>>(d, w, acc_voxels, per, choose);
   count_launch();
   return cudaPeekAtLastError();
 }
@@ -99,8 +100,8 @@ cudaError_t L_bake_mark(const SplatDev* d, const Work* w, int blocks, BakeList l
 cudaError_t L_bake_gather(const SplatDev* d, int blocks, BakeList list, cudaStream_t st) {
   CLAY_LAUNCH(k_bake_gather, blocks, 32 * kGatherWarps, st, d, list);
 }
-cudaError_t L_resolve(const SplatDev* d, const Work* w, int blocks, cudaStream_t st) {
-  CLAY_LAUNCH(k_resolve, blocks, kResolveThreads, st, d, w);
+cudaError_t L_resolve(const SplatDev* d, const Work* w, int blocks, bool choose, cudaStream_t st) {
+  CLAY_LAUNCH(k_resolve, blocks, kResolveThreads, st, d, w, choose);
 }
 cudaError_t L_field_query_mip(const FieldDev* f, const float* pts, int n, int mip, float* sxy, float* fxy, cudaStream_t st) {
   CLAY_LAUNCH(k_field_query_mip, (n + 255) / 256, 256, st, f, pts, n, mip, sxy, fxy);

@@ -48,9 +48,10 @@ cudaError_t L_forces_team(const SceneDev* s, const Work* w, int blocks, int sub,
 // `blocks_y` = mip levels when w == nullptr.
 // acc_voxels: size of the shared-memory minimum tile (dynamic shared memory, 4 B per voxel).
 // `per`: particles per block when w == nullptr.
-cudaError_t L_splat(const SplatDev* d, const Work* w, int blocks, int blocks_y, uint32_t acc_voxels, cudaStream_t st,
+// `choose`: clouds that the device gathers (bake_gathers) are left out.
+cudaError_t L_splat(const SplatDev* d, const Work* w, int blocks, int blocks_y, uint32_t acc_voxels, bool choose, cudaStream_t st,
                     uint32_t per = 32 * kSplatWarps);
-cudaError_t L_resolve(const SplatDev* d, const Work* w, int blocks, cudaStream_t st);
+cudaError_t L_resolve(const SplatDev* d, const Work* w, int blocks, bool choose, cudaStream_t st);
 // The bake order of large scenes: parts of kSortPart bins, then blocks of 256 particles.
 cudaError_t L_sort_scan(const SceneDev* s, const SplatDev* d, const Work* w, int blocks, bool final, cudaStream_t st);
 cudaError_t L_sort_scatter(const SceneDev* s, const SplatDev* d, const Work* w, int blocks, cudaStream_t st);

@@ -75,20 +75,116 @@ def test_gathered_batch_equals_splatted_scenes(root, lanes):
         o.destroy()
 
 
-def test_gathered_surface_of_many_chunks_equals_splatted(root):
-    """A small dense scene with a surface of more than 131,072 chunks of 8^3 voxels: its super-groups are counted, and a
-    chunk's number times their 32,768 particles (which passes 2^32 there) decides nothing."""
+def mist(n, spacing, center, seed):
+    """Particles at random places of a cube, `spacing` apart on average, in no order."""
+    from clay_engine_b200.core import PARTICLE_DTYPE
+
+    p, half = np.zeros(n, PARTICLE_DTYPE), 0.5 * spacing * n ** (1 / 3)
+    p["pos"] = np.random.default_rng(seed).uniform(-half, half, (n, 3)) + center
+    return p
+
+
+def is_gathered(p, res):
+    """The rule by which the device gathers a surface that its launches let it choose for."""
+    c = np.floor((p["pos"].astype(np.float64) - ORIGIN) / 0.22).astype(np.int64)  # smoothing 2.2 x the spacing of 0.1
+    cells, occupied = int(np.prod(c.max(0) - c.min(0) + 1)), len(np.unique(c, axis=0))
+    n = len(p)
+    return n >= 8192 and (n >= 2 * cells or (8 * n >= res ** 3 and (5 * n >= 6 * cells or 5 * occupied >= 2 * cells)))
+
+
+def surface_sim(root, p, res, mips, band=3.0, capacity=None):
     import clay_engine_b200 as ce
 
-    wanted = [("pile", 8192, 8200, 416, 2), ("pile", 40000, 255000, 64, 2)]
-    assert (416 // 8) ** 3 + (208 // 8) ** 3 > 1 << 17 and sum(c for _, _, c, _, _ in wanted) >= 1 << 18
-    together, alone = make(root, "reference", wanted), make(root, "reference", wanted)
+    s = ce.FluidSim(root, None, dict(capacity=capacity or len(p), spacing=0.1, radius=0.05, substeps=1, gravity=(0, 0, 0), bakeResolution=res,
+                                     bakeMipLevels=mips, bakeBand=band, worldSize=24.0, origin=ORIGIN))
+    s.upload(p)
+    return s
+
+
+# (spacing: dense pile or mist, live, resolution, levels): around a super-group (32,768), partly filled leaves and groups, one
+# level and several, levels of 8^3
+GATHERED = [("pile", 0.1, 8192, 32, 2), ("pile", 0.1, 8193, 8, 1), ("pile", 0.1, 32768, 64, 2), ("pile", 0.1, 32769, 128, 4),
+            ("mist", 0.2, 33000, 64, 3), ("mist", 0.18, 9999, 40, 1), ("pile", 0.1, 250000, 96, 3), ("mist", 0.17, 130000, 64, 3)]
+
+
+@pytest.mark.parametrize("lanes", [1, 3, 0])
+def test_gathered_scenes_of_a_batch_equal_splatted(root, lanes):
+    """Scenes that the device gathers in a batch, and the same ones splatted by themselves (a scene alone of fewer than 2^18
+    particles is). lanes 0: step_subset."""
+    import clay_engine_b200 as ce
+    from clay_engine_b200 import scenes
+
+    clouds = []
+    for i, (kind, spacing, n, res, mips) in enumerate(GATHERED):
+        p = scenes.lattice_block(n, spacing, (0.3, 2.0, -0.7), i) if kind == "pile" else mist(n, spacing, (0.0, 5.0, 0.0), i)
+        assert is_gathered(p, res) and n < 1 << 18
+        clouds.append(p)
+    assert sum(len(p) for p in clouds) >= 3 << 17
+    together, alone = ([surface_sim(root, p, g[3], g[4], (2.0, 4.0, 3.0)[i % 3], len(p) + 5 * i) for i, (p, g) in enumerate(zip(clouds, GATHERED))]
+                       for _ in range(2))
     b = ce.Batch(root, together)
-    b.step()
+    b.set_lanes(max(lanes, 1))
+    for _ in range(2):
+        if lanes:
+            b.step()
+        else:
+            b.step_subset(list(range(len(together))))
+        for s in alone:
+            s.step()
     for i, (x, y) in enumerate(zip(together, alone)):
-        y.step()
         gd, ad = x.surface.volume.download()[0], y.surface.volume.download()[0]
-        assert np.array_equal(gd, ad), f"scene {i}: {(gd != ad).sum()} voxels differ"
+        assert np.array_equal(gd, ad), f"scene {i} {GATHERED[i]}: {(gd != ad).sum()} voxels differ"
         assert (ad != 0x3C00).any()
     for o in [b] + together + alone:
+        o.destroy()
+
+
+@pytest.mark.parametrize("kind,spacing,n,res,mips,gathered", [("mist", 0.2, 1 << 18, 64, 3, True), ("mist", 0.2, 270001, 128, 2, True),
+                                                              ("pile", 0.1, 300000, 64, 3, True), ("mist", 0.2, 300000, 192, 1, False),
+                                                              ("pile", 0.09, 1 << 19, 32, 2, True), ("spray", 0.0, 300000, 64, 3, False)])
+def test_large_scene_alone_equals_splatted(root, kind, spacing, n, res, mips, gathered):
+    """A scene by itself at the sizes from which the device may choose, on either side of its rule, against its cloud baked
+    by a SplatField of its own."""
+    import torch
+
+    import clay_engine_b200 as ce
+    from clay_engine_b200 import scenes
+
+    p = scenes.lattice_block(n, spacing, (0.0, 4.0, 0.0), n) if kind == "pile" else mist(n, spacing, (0.0, 6.0, 0.0), n)
+    if kind == "spray":  # a pile, and a tenth of it as a thin spray over the world
+        p = scenes.lattice_block(n, 0.1, (0.0, 1.0, 0.0), n)
+        p["pos"][::10] = np.random.default_rng(n).uniform((-11, -3, -11), (11, 19, 11), (len(p[::10]), 3))
+    assert is_gathered(p, res) == gathered
+    sim = surface_sim(root, p, res, mips)
+    for _ in range(2):
+        sim.step()
+    now = torch.from_numpy(np.ascontiguousarray(sim.download()["pos"])).cuda()
+    splat = ce.SplatField(root, ce.ParticleCloud(n, now), radius=0.1 * 1.1, resolution=res, mipLevels=mips, band=3.0, worldSize=24.0,
+                          origin=ORIGIN)
+    splat.bake()
+    gd, ad = sim.surface.volume.download()[0], splat.volume.download()[0]
+    assert np.array_equal(gd, ad), f"{(gd != ad).sum()} voxels differ"
+    assert (ad != 0x3C00).any()
+    for o in (sim, splat):
+        o.destroy()
+
+
+def test_gathered_surface_of_many_chunks_equals_splatted(root):
+    """A dense scene with a surface of more than 131,072 chunks of 8^3 voxels: its super-groups are counted, and a chunk's
+    number times their 32,768 particles (which passes 2^32 there) decides nothing."""
+    import clay_engine_b200 as ce
+    from clay_engine_b200 import scenes
+
+    assert (416 // 8) ** 3 + (208 // 8) ** 3 > 1 << 17
+    clouds = [scenes.lattice_block(n, 0.1, (0.3, 2.0, -0.7), n) for n in (9000, 400000)]
+    assert is_gathered(clouds[0], 416)
+    together = [surface_sim(root, p, r, 2) for p, r in zip(clouds, (416, 64))]
+    alone = surface_sim(root, clouds[0], 416, 2)
+    b = ce.Batch(root, together)
+    b.step()
+    alone.step()
+    gd, ad = together[0].surface.volume.download()[0], alone.surface.volume.download()[0]
+    assert np.array_equal(gd, ad), f"{(gd != ad).sum()} voxels differ"
+    assert (ad != 0x3C00).any()
+    for o in [b, alone] + together:
         o.destroy()
