@@ -3604,8 +3604,9 @@ __global__ void __launch_bounds__(kExtractThreads) k_ext_cells(const ExtractDev*
       sum += d[i];
     }
     float ax = 0.0f, ay = 0.0f, az = 0.0f, aw = 0.0f;
-    // no edge crosses where no two corners differ in sign (a sum that is not a number: see for each)
-    if (!(low >= 0.0f) && !(high <= 0.0f) || sum != sum) {
+    // no edge crosses where no two corners differ in sign; a sum that is not finite: see for each (the product of a zero and
+    // an infinite end is not a number, which crosses)
+    if (!(low >= 0.0f) && !(high <= 0.0f) || !(fabsf(sum) < __int_as_float(0x7f800000))) {
     // the twelve edges in the reference's order
     ext_cross(x0, y0, z0, d0, x1, y0, z0, dx, ax, ay, az, aw);
     ext_cross(x0, y1, z0, dy, x1, y1, z0, dxy, ax, ay, az, aw);

@@ -176,3 +176,29 @@ def test_lattice_sizes_are_bit_exact(root, oracle, res):
     assert res < 7 or counts[0] > 50
     x.destroy()
     vol.destroy()
+
+
+def test_zero_beside_infinite_distances(root, oracle):
+    """Cells whose corners lie at zero and at infinity (a volume so large that its distances overflow) and at nothing else:
+    their product is not a number, so that those edges cross (extract.ts:262-278 tests da * db >= 0), at the zero end."""
+    import clay_engine_b200 as ce
+
+    res, world, origin = 16, 1e38, (-5e37, -5e37, -5e37)
+    dist = np.zeros((res, res, res), np.float16)
+    dist[:, :, 8:] = 30000.0
+    v = ce.SdfVolume(root, resolution=res, worldSize=world, origin=origin, mipLevels=1)
+    d, m = dist.reshape(-1).view(np.uint16), np.zeros(res ** 3, np.uint16)
+    v.upload(d, m)
+    f = ce.volumeField(v)
+    pset = ParticleSetDev(8000)
+    x = ce.SurfaceExtractor(root, pset.parts, 8000, pset.bodies, 1, f, 0, 0, 8000, resolution=res)
+    x.setRegion(origin, world, (0.0, 0.0, 0.0), False)
+    x.extract()
+    tri, draw = x.indices()
+    hp, hb = ParticleSetDev(8000).host()
+    idx, odraw, cnt = oracle.extract(oracle.make_field([oracle.VolumeData(res, 1, origin, world, 4.0, dist=d, mat=m)]), hp, hb, res, 0, 0, 8000,
+                                     origin, world)
+    assert int(cnt[0]) > 0 and tuple(int(c) for c in cnt) == x.counts()
+    assert np.array_equal(draw, odraw) and np.array_equal(idx[: int(odraw[0])].reshape(-1, 3), tri)
+    for o in (x, f, v):
+        o.destroy()
