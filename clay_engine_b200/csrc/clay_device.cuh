@@ -383,8 +383,7 @@ __device__ __forceinline__ float texel(const Vol& v, int x, int y, int z) {
 // Texels x0 and x1 (the same one or the next) of a row, for scattered points: those are bound by the lines
 // that L1 looks up, one a lane and load, so both come with the aligned 8 bytes around x0 (rows are
 // multiples of 8 texels, planes and levels 16-byte aligned), and with a second load where x1 begins the
-// next four. Points whose neighbours share lines are better served by a load per texel
-// (surface nets on 128^3: 378 us against 472, with 16 bytes around x0).
+// next four. Points whose neighbours share lines are bound by instructions, and a load per texel takes fewer.
 __device__ __forceinline__ void texel_pair(const __half* __restrict__ row, int x0, int x1, float& a, float& b) {
   const uint2 w = __ldg(reinterpret_cast<const uint2*>(row + (x0 & ~3)));
   auto pick = [&](int i) {
@@ -407,7 +406,23 @@ __device__ __forceinline__ void tri_axis(float u, int R, int& i0, int& i1, float
 
 __device__ __forceinline__ float lerpf(float a, float b, float f) { return a + (b - a) * f; }
 
-template <bool kScattered = false>
+// Where a point falls between the texels of a level.
+struct TriAt {
+  int x0, x1, y0, y1, z0, z1;
+  float fx, fy, fz;
+  __device__ __forceinline__ TriAt(const Vol& v, float px, float py, float pz) {
+    tri_axis(__fdiv_rn(px - v.ox, v.extent), v.res, x0, x1, fx);
+    tri_axis(__fdiv_rn(py - v.oy, v.extent), v.res, y0, y1, fy);
+    tri_axis(__fdiv_rn(pz - v.oz, v.extent), v.res, z0, z1, fz);
+  }
+  // `along_x(y, z)`: the value at fx on the row (y, z).
+  template <class F>
+  __device__ __forceinline__ float mix(F&& along_x) const {
+    const float c00 = along_x(y0, z0), c10 = along_x(y1, z0), c01 = along_x(y0, z1), c11 = along_x(y1, z1);
+    return lerpf(lerpf(c00, c10, fy), lerpf(c01, c11, fy), fz);
+  }
+};
+
 __device__ __forceinline__ float trilinear(const Vol& v, float px, float py, float pz) {
   float ux = __fdiv_rn(px - v.ox, v.extent);
   float uy = __fdiv_rn(py - v.oy, v.extent);
@@ -417,16 +432,44 @@ __device__ __forceinline__ float trilinear(const Vol& v, float px, float py, flo
   tri_axis(ux, v.res, x0, x1, fx);
   tri_axis(uy, v.res, y0, y1, fy);
   tri_axis(uz, v.res, z0, z1, fz);
-  auto along_x = [&](int y, int z) {
-    if constexpr (!kScattered) return lerpf(texel(v, x0, y, z), texel(v, x1, y, z), fx);
-    float a, b;
-    texel_pair(v.dist + static_cast<size_t>(v.res) * (static_cast<size_t>(y) + static_cast<size_t>(v.res) * z), x0, x1, a, b);
-    return lerpf(a, b, fx);
-  };
-  const float c00 = along_x(y0, z0), c10 = along_x(y1, z0), c01 = along_x(y0, z1), c11 = along_x(y1, z1);
+  float c00 = lerpf(texel(v, x0, y0, z0), texel(v, x1, y0, z0), fx);
+  float c10 = lerpf(texel(v, x0, y1, z0), texel(v, x1, y1, z0), fx);
+  float c01 = lerpf(texel(v, x0, y0, z1), texel(v, x1, y0, z1), fx);
+  float c11 = lerpf(texel(v, x0, y1, z1), texel(v, x1, y1, z1), fx);
   float c0 = lerpf(c00, c10, fy);
   float c1 = lerpf(c01, c11, fy);
   return lerpf(c0, c1, fz);
+}
+
+// The same of two planes of a level, for points of which nothing is known: a row's texels as a pair where the rows of the warp's
+// points lie more than kRowsNear apart, else a load each. 4,096,000 points at 192^3 (all as pairs, all by themselves):
+// random 143 and 166 us, along z 171 and 256, a lattice's in order 78 and 80; at 24^3 80 and 94, 74 and 68, 74 and 68. Chosen by
+// the warp 136, 168, 66; 76, 64, 64.
+constexpr int kRowsNear = 6;
+__device__ __forceinline__ void trilinear_planes(const Vol& v, const __half* __restrict__ first, const __half* __restrict__ second,
+                                                 float px, float py, float pz, float& a, float& b) {
+  const TriAt t(v, px, py, pz);
+  const uint32_t on = __activemask();
+  const int apart = (__reduce_max_sync(on, t.y0) - __reduce_min_sync(on, t.y0)) + (__reduce_max_sync(on, t.z0) - __reduce_min_sync(on, t.z0));
+  auto row = [&](const __half* __restrict__ p, int y, int z) {
+    return p + static_cast<size_t>(v.res) * (static_cast<size_t>(y) + static_cast<size_t>(v.res) * z);
+  };
+  if (apart > kRowsNear) {  // the branch around all loads, so that they are issued together
+    auto along_x = [&](const __half* __restrict__ p, int y, int z) {
+      float lo, hi;
+      texel_pair(row(p, y, z), t.x0, t.x1, lo, hi);
+      return lerpf(lo, hi, t.fx);
+    };
+    a = t.mix([&](int y, int z) { return along_x(first, y, z); });
+    b = t.mix([&](int y, int z) { return along_x(second, y, z); });
+  } else {
+    auto along_x = [&](const __half* __restrict__ p, int y, int z) {
+      const __half* __restrict__ r = row(p, y, z);
+      return lerpf(__half2float(__ldg(r + t.x0)), __half2float(__ldg(r + t.x1)), t.fx);
+    };
+    a = t.mix([&](int y, int z) { return along_x(first, y, z); });
+    b = t.mix([&](int y, int z) { return along_x(second, y, z); });
+  }
 }
 
 __device__ __forceinline__ void vol_sample(const Vol& v, float px, float py, float pz, float& sx, float& sy) {
@@ -545,10 +588,8 @@ __device__ __forceinline__ void leaf_sample_mip(const LeafDev& lf, float px, flo
   float bw;
   vol_level(lf.vp, mip, off, R, bw);
   v.res = R;
-  v.dist = lf.vp->dist + off;
-  const float raw = trilinear<true>(v, qx, qy, qz);
-  v.dist = lf.vp->mat + off;
-  fy = trilinear<true>(v, qx, qy, qz);
+  float raw;
+  trilinear_planes(v, lf.vp->dist + off, lf.vp->mat + off, qx, qy, qz, raw, fy);
   sx = raw * bw;
   sy = raw;
 }
@@ -4226,8 +4267,7 @@ __global__ void k_field_query(const FieldDev* __restrict__ f, const float* __res
 }
 
 // Collider query at a level: sample(p, mip) and field(p, mip) at n points. Bound by the sectors that scattered
-// points fetch (two planes, four rows each): 4,194,304 of them at 192^3 took 174 us with a load per texel,
-// now 150.
+// points fetch (two planes, four rows each).
 __global__ void __launch_bounds__(256, 5) k_field_query_mip(const FieldDev* __restrict__ f, const float* __restrict__ pts, int n,
                                                             int mip, float* __restrict__ sxy, float* __restrict__ fxy) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;

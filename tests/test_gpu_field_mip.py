@@ -111,3 +111,31 @@ def test_rows_of_texels_end_to_end(root, shift):
         s, f = field.query_mip(pts, mip)
         assert np.array_equal(out[0].cpu().numpy(), s) and np.array_equal(out[1].cpu().numpy(), f)
         assert len(np.unique(s[:, 1])) > 20
+
+
+@pytest.mark.parametrize("order", ["lattice", "along z", "scattered"])
+def test_order_of_the_points(root, oracle, order):
+    """Level sampling reads rows as pairs of texels or texel by texel, by how far apart the rows of a warp's points lie: the
+    same points in the order of a lattice, along z, and in none, some of them outside the volume."""
+    import clay_engine_b200 as ce
+
+    v = ce.SdfVolume(root, resolution=64, worldSize=8.0, origin=(-4.0, -4.0, -4.0))
+    v.build(np.concatenate([brushes.make_brush("box", pos=(0, -2.5, 0), size=(3.5, 0.5, 3.5), material=0.3),
+                            brushes.make_brush("sphere", pos=(1, -1, 0.5), size=1.2, material=0.6)]))
+    d, m = v.download()
+    of = oracle.make_field([oracle.VolumeData(64, v.mipLevels, (-4.0, -4.0, -4.0), 8.0, v.band, dist=d, mat=m)])
+    a = np.linspace(-4.3, 4.3, 37, dtype=np.float32)
+    z, y, x = np.meshgrid(a, a, a, indexing="ij")
+    pts = np.stack([x.ravel(), y.ravel(), z.ravel()], 1)
+    if order == "along z":
+        pts = np.ascontiguousarray(pts.reshape(37, 37, 37, 3).transpose(2, 1, 0, 3)).reshape(-1, 3)
+    if order == "scattered":
+        pts = pts[np.random.default_rng(3).permutation(len(pts))]
+    f = ce.volumeField(v)
+    for mip in range(v.mipLevels):
+        gs, gf = f.query_mip(pts, mip)
+        os_, of_ = oracle.field_query_mip_f32(of, pts, mip)
+        assert np.array_equal(gs.view(np.uint32), os_.view(np.uint32)), mip
+        assert np.array_equal(gf.view(np.uint32), of_.view(np.uint32)), mip
+    f.destroy()
+    v.destroy()
