@@ -121,8 +121,9 @@ struct __align__(16) GridState {
   uint32_t L;  // bbox cells; local index L is the out-of-grid bucket
   int32_t x0, y0, z0;
   uint32_t bx, by, bz;
-  // of the last substep, counted where the scene may be gathered: cells of the box that hold a particle, particles outside the grid
-  uint32_t occupied, outside;
+  // of the last substep, counted where the scene may be gathered: cells of the box that hold a particle, runs of 128 cells
+  // that do, particles outside the grid
+  uint32_t occupied, runs, outside;
   uint32_t part_sum[kMaxParts];
 };
 
@@ -739,6 +740,7 @@ __global__ void k_cell_key(const SceneDev* __restrict__ scenes, const Work* __re
     S.contacts->count = 0u;
     S.gs->overflow = 0u;
     S.gs->occupied = 0u;
+    S.gs->runs = 0u;
   }
   uint32_t lo[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu};
   uint32_t hinv[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu};
@@ -879,7 +881,7 @@ __global__ void __launch_bounds__(1024, 2) k_scan_final(const SceneDev* __restri
   scan_part(S, w.sub, n, beg, end);
   if (beg >= end) return;
   __shared__ uint32_t s_off;
-  __shared__ uint32_t s_warp[32];
+  __shared__ uint32_t s_warp[32], s_runs[32];
   if (threadIdx.x < 32) {
     uint32_t o = 0;
     for (uint32_t q = threadIdx.x; q < w.sub; q += 32u) o += gs->part_sum[q];
@@ -887,13 +889,14 @@ __global__ void __launch_bounds__(1024, 2) k_scan_final(const SceneDev* __restri
     if (threadIdx.x == 0) s_off = o;
   }
   __syncthreads();
-  uint32_t run = s_off, occupied = 0;
+  uint32_t run = s_off, occupied = 0, runs = 0;
   const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (uint32_t c0 = beg; c0 < end; c0 += 4u * blockDim.x) {
     const uint32_t c = c0 + 4u * threadIdx.x;
     const uint4 q = c < end ? scan_counts(S, c, end) : make_uint4(0u, 0u, 0u, 0u);
     const uint32_t v = (q.x + q.y) + (q.z + q.w);
     occupied += (q.x != 0u) + (q.y != 0u) + (q.z != 0u) + (q.w != 0u);
+    runs += __any_sync(0xffffffffu, v != 0u);
     uint32_t x = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -933,10 +936,13 @@ __global__ void __launch_bounds__(1024, 2) k_scan_final(const SceneDev* __restri
   // for bake_gathers: the occupied cells (with the particles outside the grid as one more)
   if (substep + 1 == S.substeps && work_count(S) >= (work ? kGatherMin : kGatherAlone)) {
     s_warp[wid] = __reduce_add_sync(0xffffffffu, occupied);
+    s_runs[wid] = runs;
     __syncthreads();
     if (wid == 0) {
       const uint32_t all = __reduce_add_sync(0xffffffffu, lane < nw ? s_warp[lane] : 0u);
+      const uint32_t held = __reduce_add_sync(0xffffffffu, lane < nw ? s_runs[lane] : 0u);
       if (lane == 0 && all) atomicAdd(&S.gs->occupied, all);
+      if (lane == 0 && held) atomicAdd(&S.gs->runs, held);
       if (lane == 0 && end == n) S.gs->outside = run - S.cell_start[n - 1u];
     }
   }
@@ -1738,19 +1744,20 @@ __device__ __forceinline__ uint32_t enc_key(float sd, float bw) {
 // Whether a fluid's surface is gathered. A splat's particle costs the voxels of its band (splat.ts:238-246: 300 to 400
 // a level), most where particles lie so far apart that each walks its own; a gather's voxel costs a descent, most where
 // boxes of 32 particles are large for the voxels. So the gather wins where the fluid fills its box: two particles a
-// cell, or, as long as there is one for eight voxels of the finest level, 1.2 a cell, or two in five cells occupied.
-// Measured over pools with a share of spray from none to nine tenths, clouds, balls, columns, layers, blobs far apart, a
-// pool with a spray up to the sky, on 32^3 to 192^3, scenes of 262,144 to 1,000,000 by themselves: 285 of 375
-// frames are gathered, 1.30 times faster on average (0.94 at worst: one layer, 119 a cell); what is left to the splat would take
-// up to 2.9 times as long by the gather (a pool of 259,000 and 2,600 in the sky, 192^3: 699 -> 2,000 us). In batches
+// cell, or, as long as there is one for eight voxels of the finest level, 1.2 a cell, or a third of the cells occupied in
+// those runs of 128 that hold any (the box of a pool under a falling stream is mostly air).
+// Measured over pools with a share of spray from none to nine tenths, without and with a stream, clouds, balls, columns,
+// layers, blobs far apart, a pool with a spray up to the sky, on 32^3 to 192^3: scenes of 262,144 to 1,000,000 by themselves
+// are gathered 1.25 times faster on average (0.94 at worst: one layer, 119 a cell), those left to the splat would
+// take up to 2.9 times as long by the gather (a pool of 259,000 and 2,600 in the sky, 192^3: 699 -> 2,000 us). In batches
 // of 393,216 and more 1.19 times (0.96 at worst). Particles outside the grid are in no order (one bin), and 7 % of them took a
 // cloud of 600,000 from 1,930 to 2,930 us: more than 1 in 64 are splatted.
 __device__ __forceinline__ bool bake_gathers(const SplatDev& D) {
   if (!D.gs) return false;
   const uint64_t n = min(*D.live_count, D.capacity), r = static_cast<uint64_t>(D.r[0]);
-  const uint64_t cells = D.gs->L, occupied = D.gs->occupied;
+  const uint64_t cells = D.gs->L, occupied = D.gs->occupied, held = min(static_cast<uint64_t>(128) * D.gs->runs, cells);
   if (n < kGatherMin || cells == 0 || 64ull * D.gs->outside > n) return false;
-  return n >= 2 * cells || (8 * n >= r * r * r && (5 * n >= 6 * cells || 5 * occupied >= 2 * cells));
+  return n >= 2 * cells || (8 * n >= r * r * r && (5 * n >= 6 * cells || 3 * occupied >= held));
 }
 
 __device__ __forceinline__ bool cloud_live(const SplatDev& D, uint32_t idx, uint32_t& i) {

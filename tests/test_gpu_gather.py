@@ -87,9 +87,11 @@ def mist(n, spacing, center, seed):
 def is_gathered(p, res):
     """The rule by which the device gathers a surface that its launches let it choose for."""
     c = np.floor((p["pos"].astype(np.float64) - ORIGIN) / 0.22).astype(np.int64)  # smoothing 2.2 x the spacing of 0.1
-    cells, occupied = int(np.prod(c.max(0) - c.min(0) + 1)), len(np.unique(c, axis=0))
-    n = len(p)
-    return n >= 8192 and (n >= 2 * cells or (8 * n >= res ** 3 and (5 * n >= 6 * cells or 5 * occupied >= 2 * cells)))
+    box = c.max(0) - c.min(0) + 1
+    at = np.unique(np.ravel_multi_index((c - c.min(0)).T[::-1], box[::-1]))
+    n, cells, occupied = len(p), int(np.prod(box)), len(at)
+    held = min(128 * len(np.unique(at // 128)), cells)
+    return n >= 8192 and (n >= 2 * cells or (8 * n >= res ** 3 and (5 * n >= 6 * cells or 3 * occupied >= held)))
 
 
 def surface_sim(root, p, res, mips, band=3.0, capacity=None):
@@ -141,7 +143,8 @@ def test_gathered_scenes_of_a_batch_equal_splatted(root, lanes):
 
 @pytest.mark.parametrize("kind,spacing,n,res,mips,gathered", [("mist", 0.2, 1 << 18, 64, 3, True), ("mist", 0.2, 270001, 128, 2, True),
                                                               ("pile", 0.1, 300000, 64, 3, True), ("mist", 0.2, 300000, 192, 1, False),
-                                                              ("pile", 0.09, 1 << 19, 32, 2, True), ("spray", 0.0, 300000, 64, 3, False)])
+                                                              ("pile", 0.09, 1 << 19, 32, 2, True), ("spray", 0.0, 300000, 64, 3, False),
+                                                              ("stream", 0.22, 300000, 64, 3, True)])
 def test_large_scene_alone_equals_splatted(root, kind, spacing, n, res, mips, gathered):
     """A scene by itself at the sizes from which the device may choose, on either side of its rule, against its cloud baked
     by a SplatField of its own."""
@@ -154,6 +157,8 @@ def test_large_scene_alone_equals_splatted(root, kind, spacing, n, res, mips, ga
     if kind == "spray":  # a pile, and a tenth of it as a thin spray over the world
         p = scenes.lattice_block(n, 0.1, (0.0, 1.0, 0.0), n)
         p["pos"][::10] = np.random.default_rng(n).uniform((-11, -3, -11), (11, 19, 11), (len(p[::10]), 3))
+    if kind == "stream":  # a thin one falls into the mist, from as high again
+        p["pos"][:3000] = np.random.default_rng(n).normal((0.0, 14.0, 0.0), (0.1, 2.0, 0.1), (3000, 3))
     assert is_gathered(p, res) == gathered
     sim = surface_sim(root, p, res, mips)
     for _ in range(2):
