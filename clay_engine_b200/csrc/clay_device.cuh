@@ -204,13 +204,14 @@ static_assert(bake_supers(1u << 26) == 2048 && 131072u >= bake_supers(1u << 26))
 struct BakeTreeLayout {
   uint64_t leaf, group, super, cursor, list, total;
 };
-// A fluid's surface may be gathered (see bake_gathers) from kGatherMin particles on, in a scene by itself from
-// kGatherAlone, in scenes of a batch when they hold kGatherBatch together: below, the gather's launches and the latency
+// A fluid's surface may be gathered (see bake_gathers) from kGatherMin particles on (twice as many into less than 64^3), in
+// a scene by itself from kGatherAlone, in scenes of a batch when they hold kGatherBatch together: below, the gather's launches and the latency
 // of its descents cost more than the splat. Dense scenes, splat and gather, a frame of one substep: by itself, 131,072
 // particles as a pool 161 and 171 us (32^3 x 2), as a ball 182 and 200 (64^3 x 3), 262,144 268 and 255, 309 and 284; as two
 // layers each in a batch, 100 scenes of 4,096 366 and 398 us (32^3 x 2), 8 of 32,768 245 and 275, 12 343 and 357, 64 of
-// 8,192 431 and 423.
-constexpr uint32_t kGatherMin = 8192, kGatherAlone = 1u << 18, kGatherBatch = 3u << 17;
+// 8,192 431 and 423; 96 uneven pools of 1,024 to 65,536 (64^3 x 3, two substeps) 2,009 us gathered from 8,192 on, 1,993 from
+// 4,096, 2,005 from 1,024.
+constexpr uint32_t kGatherMin = 4096, kGatherAlone = 1u << 18, kGatherBatch = 3u << 17;
 // Scenes of more particles than kSortMin are baked in Morton order (see k_sort_scan): at most kSortBins
 // bins, scanned in parts.
 constexpr uint32_t kSortMin = 8192, kSortBins = 1u << 18, kSortPart = 2048, kSortParts = kSortBins / kSortPart + 1;
@@ -1756,7 +1757,7 @@ __device__ __forceinline__ bool bake_gathers(const SplatDev& D) {
   if (!D.gs) return false;
   const uint64_t n = min(*D.live_count, D.capacity), r = static_cast<uint64_t>(D.r[0]);
   const uint64_t cells = D.gs->L, occupied = D.gs->occupied, held = min(static_cast<uint64_t>(128) * D.gs->runs, cells);
-  if (n < kGatherMin || cells == 0 || 64ull * D.gs->outside > n) return false;
+  if (n < (r < 64 ? 2 * kGatherMin : kGatherMin) || cells == 0 || 64ull * D.gs->outside > n) return false;
   return n >= 2 * cells || (8 * n >= r * r * r && (5 * n >= 6 * cells || 3 * occupied >= held));
 }
 

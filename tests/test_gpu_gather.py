@@ -91,7 +91,7 @@ def is_gathered(p, res):
     at = np.unique(np.ravel_multi_index((c - c.min(0)).T[::-1], box[::-1]))
     n, cells, occupied = len(p), int(np.prod(box)), len(at)
     held = min(128 * len(np.unique(at // 128)), cells)
-    return n >= 8192 and (n >= 2 * cells or (8 * n >= res ** 3 and (5 * n >= 6 * cells or 3 * occupied >= held)))
+    return n >= (4096 if res >= 64 else 8192) and (n >= 2 * cells or (8 * n >= res ** 3 and (5 * n >= 6 * cells or 3 * occupied >= held)))
 
 
 def surface_sim(root, p, res, mips, band=3.0, capacity=None):
@@ -105,7 +105,7 @@ def surface_sim(root, p, res, mips, band=3.0, capacity=None):
 
 # (spacing: dense pile or mist, live, resolution, levels): around a super-group (32,768), partly filled leaves and groups, one
 # level and several, levels of 8^3
-GATHERED = [("pile", 0.1, 8192, 32, 2), ("pile", 0.1, 8193, 8, 1), ("pile", 0.1, 32768, 64, 2), ("pile", 0.1, 32769, 128, 4),
+GATHERED = [("pile", 0.1, 4096, 64, 2), ("pile", 0.1, 8192, 32, 2), ("pile", 0.1, 8193, 8, 1), ("pile", 0.1, 32768, 64, 2), ("pile", 0.1, 32769, 128, 4),
             ("mist", 0.2, 33000, 64, 3), ("mist", 0.18, 9999, 40, 1), ("pile", 0.1, 250000, 96, 3), ("mist", 0.17, 130000, 64, 3)]
 
 
