@@ -3322,11 +3322,10 @@ __global__ void __launch_bounds__(256) k_build(const BuildDev B, const BrushDev*
   }
   const uint32_t kept = __ballot_sync(0xffffffffu, keep);
   if (lane == 0) s_warp[wid] = __popc(kept);
-  __syncthreads();
-  uint32_t before = 0, all = 0;
-  for (uint32_t k = 0; k < 8; k++) {
-    if (k < wid) before += s_warp[k];
-    all += s_warp[k];
+  uint32_t before = 0;
+  if (nbrush > 32) {  // else the first warp alone has any
+    __syncthreads();
+    for (uint32_t k = 0; k < wid; k++) before += s_warp[k];
   }
   const uint32_t place = before + __popc(kept & ((1u << lane) - 1u));
   if (keep && place < kBuildKeep) {
@@ -3334,6 +3333,9 @@ __global__ void __launch_bounds__(256) k_build(const BuildDev B, const BrushDev*
     s_inv[place] = __frcp_rn(fmaxf(s_brush[place].scale, 1e-5f));
   }
   __syncthreads();
+  uint32_t all = s_warp[0];
+  if (nbrush > 32)
+    for (uint32_t k = 1; k < 8; k++) all += s_warp[k];
   const uint32_t n = min(all, kBuildKeep);
   const int lx = threadIdx.x & 7, ly = (threadIdx.x >> 3) & 7, lz2 = threadIdx.x >> 6;
   for (int half = 0; half < 2; half++) {
