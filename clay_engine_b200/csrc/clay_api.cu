@@ -64,7 +64,9 @@ namespace {
   } while (0)
 
 constexpr int TILE = 8;
-constexpr int64_t kDiscsLeast = 16, kDiscBlocks = 148 * 8;  // discs per block at least, blocks wanted at most
+// Discs per block at least, blocks wanted at most, and blocks of 256 from which discs of a narrow band (below three voxels)
+// stay in them: a block's set-up then costs more than its discs' walks.
+constexpr int64_t kDiscsLeast = 16, kDiscBlocks = 148 * 6, kDiscNarrow = 148 * 2;
 constexpr int kMaxBrushes = 256;  // one per thread of the build's cull
 constexpr int kMaxResolution = 4096;  // 4096^3 voxels per level: far beyond device memory, far below int64 overflow
 
@@ -619,10 +621,12 @@ void free_splat(clay_splat* s) {
 // Chunks of 8^3 voxels over all levels, in blocks of the mark pass.
 int mark_blocks(const clay_splat* s) { return static_cast<int>((s->vol->total / 512 + kMarkChunks - 1) / kMarkChunks); }
 
-// Discs per block of the splat, given the blocks that so many make.
+// Discs per block of the splat, given the blocks that so many make and the widest band. 60,000 discs into 32^3 x 2, band 2: 97 us
+// in blocks of 256 (470 of them), 111 in 128, band 4: 304 and 283; 20,000, band 2: 75 and 53 (in 32), band 4: 229 and 121.
 template <class Blocks>
-int64_t discs_per_block(Blocks&& blocks) {
+int64_t discs_per_block(double band, Blocks&& blocks) {
   int64_t per = kSplatThreads;
+  if (band < 3 && blocks(per) >= kDiscNarrow) return per;
   while (per > kDiscsLeast && blocks(per) < kDiscBlocks) per /= 2;
   return per;
 }
@@ -652,7 +656,7 @@ int splat_bake(clay_splat* s, cudaStream_t st, const SceneDev* scene, int64_t it
   const SplatDev* d = scene ? s->d_ordered : s->d;
   if (n > 0) {
     // a small disc cloud in blocks of fewer particles, until they fill the device (see k_splat)
-    const int64_t per = s->cloud.normals ? discs_per_block([&](int64_t p) { return (n + p - 1) / p * s->mips; }) : kSplatThreads;
+    const int64_t per = s->cloud.normals ? discs_per_block(s->band, [&](int64_t p) { return (n + p - 1) / p * s->mips; }) : kSplatThreads;
     int blocks = static_cast<int>((n + per - 1) / per);
     CK(L_splat(d, nullptr, blocks, s->mips, s->cloud.normals ? kSplatAccVoxelsDiscs : kSplatAccVoxels, choose, st,
                static_cast<uint32_t>(per)));
@@ -1740,7 +1744,9 @@ int batch_build(clay_batch* b) {
     for (size_t i = 0; i < all.size(); i++) all[i] = static_cast<int>(i);
     b->gather = b->gather && batch_list(b, all).items;  // clay_batch_profile steps them in one lane
   }
-  const int64_t disc_block = discs_per_block([&](int64_t p) {  // the bodies of the batch together
+  double band = 0;
+  for (const clay_splat* x : b->extra) band = std::max(band, x->band);
+  const int64_t disc_block = discs_per_block(band, [&](int64_t p) {  // the bodies of the batch together
     int64_t n = 0;
     for (const clay_splat* x : b->extra) n += (x->cloud.capacity + p - 1) / p * x->mips;
     return n;
