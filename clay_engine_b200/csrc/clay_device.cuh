@@ -200,9 +200,10 @@ constexpr uint32_t kLeafN = 32, kGroupN = 32 * kLeafN, kSuperN = 32 * kGroupN;
 __host__ __device__ constexpr uint32_t bake_supers(uint32_t n) { return (n + kSuperN - 1) / kSuperN; }
 static_assert(bake_supers(1) == 1 && bake_supers(kSuperN) == 1 && bake_supers(kSuperN + 1) == 2);
 static_assert(bake_supers(1u << 26) == 2048 && 131072u >= bake_supers(1u << 26));  // such a chunk writes none
-// Scratch of the tree of `n` particles, in 16-byte units, and where its parts start.
+// Scratch of the tree of `n` particles, in 16-byte units: where its parts start after the positions, the last of them the bake
+// list where there is room for one (clay_splat::list).
 struct BakeTreeLayout {
-  uint64_t leaf, group, super, cursor, list, total;
+  uint64_t leaf, group, super, cursor, list;
 };
 // A fluid's surface may be gathered (see bake_gathers) from kGatherMin particles on (twice as many into less than 64^3), in
 // a scene by itself from kGatherAlone, in scenes of a batch when they hold kGatherBatch together: below, the gather's launches and the latency
@@ -215,16 +216,19 @@ constexpr uint32_t kGatherMin = 4096, kGatherAlone = 1u << 18, kGatherBatch = 3u
 // Scenes of more particles than kSortMin are baked in Morton order (see k_sort_scan): at most kSortBins
 // bins, scanned in parts.
 constexpr uint32_t kSortMin = 8192, kSortBins = 1u << 18, kSortPart = 2048, kSortParts = kSortBins / kSortPart + 1;
-__host__ __device__ inline BakeTreeLayout bake_tree_layout(uint64_t n) {
-  BakeTreeLayout l;
+__host__ __device__ constexpr BakeTreeLayout bake_tree_layout(uint64_t n) {
+  BakeTreeLayout l{};
   l.leaf = (n + kLeafN - 1) / kLeafN * kLeafN;  // the positions, padded to whole leaves
   l.group = l.leaf + 2 * ((n + kLeafN - 1) / kLeafN);
   l.super = l.group + 2 * ((n + kGroupN - 1) / kGroupN);
   l.cursor = l.super + 2 * ((n + kSuperN - 1) / kSuperN);
   l.list = l.cursor + (n > kSortMin ? (kSortBins + 1 + kSortParts + 3) / 4 : 0);
-  l.total = l.list;  // the list of a scene gathered by itself follows: see bake_list_fits
   return l;
 }
+// The tree lies in a scene's neighbour lists (16 bytes for 4 of kMaxNbr entries a particle), which no pass reads any
+// more when the surface is baked: most in need are the smallest scene and the smallest that is sorted.
+constexpr bool bake_tree_fits(uint64_t n) { return bake_tree_layout(n).list <= n * (kMaxNbr / 4); }
+static_assert(bake_tree_fits(kGatherMin) && bake_tree_fits(kSortMin + 1));
 // The blocks of 8 x 4 x 2 voxels within reach of a cloud, as (object | level << 28, block index in
 // its level), from the front those taken eight voxels at a time, from the back the others; and the
 // counters: how many at the front, how many tickets the gather pass has drawn, how many at the back.
@@ -3513,14 +3517,8 @@ __device__ __forceinline__ void ext_origin(const ExtractDev& E, float& ox, float
   }
 }
 
-__device__ __forceinline__ float ext_dist(const ExtractDev& E, float px, float py, float pz) {
-  float sx = 0.0f, sy = 0.0f;
-  if (E.field->n > 0) field_pick(E.field, px, py, pz, sx, sy);
-  return sx;
-}
-
 // The field's distances at a cell's eight corners (x0 or x1, y0 or y1, z0 or z1; corner i takes bit 0, 1, 2 of i),
-// the same operations as ext_dist at each: what depends on one axis alone (the offset, the box test's term, the
+// the same operations as field_pick at each: what depends on one axis alone (the offset, the box test's term, the
 // division by the extent, the texel indices and the fraction) is done once per axis and end instead of at
 // every corner.
 __device__ __forceinline__ void ext_corners(const ExtractDev& E, const float (&px)[2], const float (&py)[2], const float (&pz)[2],
