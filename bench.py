@@ -438,11 +438,11 @@ def measure_next_rows(root, stream, threads):
         hbody = np.zeros(1, scenes.BODY_RECORD)
         cs = _cpu_s(lambda: oracle.extract(sofield, hpart, hbody, res, 0, 0, cap, bo, box))
         ext[str(res)] = {"cells": res ** 3, "particles": nv, "ms_per_extract": ms, "value": res ** 3 / (ms / 1e3),
-                         "achieved_gbs": (nv * 96 + res ** 3 * 36) / (ms / 1e3) / 1e9, "cpu_value": res ** 3 / cs}
+                         "achieved_gbs": (nv * 128 + res ** 3 * 5) / (ms / 1e3) / 1e9, "cpu_value": res ** 3 / cs}
         x.destroy()
     out["extract"] = {"workload": "surface nets of the clay-body sphere (r 0.95) over its 2.656 m box",
-                      "unit": "lattice cells/s", "bytes": "96 B per particle + 36 B scratch per cell",
-                      "bound": "field samples (8 + 9 per vertex cell, 4 per lattice point)", "lattices": ext,
+                      "unit": "lattice cells/s", "bytes": "96 B record and 32 B scratch per particle + 5 B scratch per cell",
+                      "bound": "field samples (8 per cell, 9 per vertex cell)", "lattices": ext,
                       "cpu_baseline": {"unit": "lattice cells/s", "cores": 1, "kind": "port", "sample": "the same"}}
 
     # 4. ClaySolver: 86 clay bodies (config 3's shell, 3,800 particles each) over a config-3
@@ -848,13 +848,14 @@ def main():
                      "algorithmic_bytes_per_launch": splat_bytes, "avg_launch_ms": round(splat_ms, 4)})
     # compute roofline (the kernels are issue-bound): algorithmic FP32 operations of the
     # reference's work per second against the FP32 lane-issue peak. The bake: 9 per in-band pair
-    # (3 sub, 3 mul, 2 add, 1 compare); k_density: 9 per candidate + 13 per accepted pair (the
+    # (3 sub, 3 mul, 2 add, 1 compare), a speed in the reference's pairs and no utilisation, since the
+    # gather leaves most of them out; k_density: 9 per candidate + 13 per accepted pair (the
     # kernel term and the sum), over both substeps (the census counts the last one)
     comp = {"unit": "FP32 lane-ops/s", "peak": lane_peak, "peak_source": f"{sms} SMs x 128 lanes x {mhz:.0f} MHz"}
     if splat_ms:
         ops = 9 * pairs
         comp["surface_bake"] = {"pairs": pairs, "pairs_per_s": pairs / (splat_ms / 1000), "ops_per_pair": 9,
-                           "frac": ops / (splat_ms / 1000) / lane_peak}
+                                "reference_pairs_vs_peak": ops / (splat_ms / 1000) / lane_peak}
     body_ms = prof.get("body_splat", (None, 0))[0]
     if body_ms and body_pairs:
         comp["k_splat_bodies"] = {"pairs": body_pairs, "pairs_per_s": body_pairs / (body_ms / 1000),

@@ -3293,10 +3293,10 @@ __device__ __forceinline__ void apply_brush(float& ax, float& ay, const BrushDev
 }
 
 // A block per 8^3 tile, all levels in one launch, the coarsest first (their tiles meet the most
-// brushes). The cull tests a brush per thread (one thread testing 64 brushes one after another was most
-// of a coarse level: 51-76 us each, at any size), keeps the first 64 in order, and the kept records
-// are folded from shared memory. Bound by the fold's FP32 work: 192^3 x 4 levels from 64 brushes, a call with
-// its upload and wait: 323 us before, 100 now.
+// brushes). The cull tests a brush per thread, keeps the first 64 in order, and the kept records are folded from shared
+// memory. Bound by the fold's FP32 work: 192^3 x 4 levels from 64 brushes, a call with its upload and wait, takes 99 us,
+// with one thread of a tile testing all brushes and a launch per level 323 (a coarse level 51-76 each, at any size); from one
+// brush, one level, 55 either way.
 __global__ void __launch_bounds__(256) k_build(const BuildDev B, const BrushDev* __restrict__ brushes, int nbrush) {
   __shared__ BrushDev s_brush[kBuildKeep];
   __shared__ float s_inv[kBuildKeep];
@@ -4052,9 +4052,9 @@ __global__ void __launch_bounds__(kSolveThreads) k_pbd_kick(const SolveDev* __re
 // out of the world, plasticity letting the rest shape follow) and finalize (pbd.ts:342-372: first-order
 // velocity, damping, speed cap). Each works on one particle's record alone, so a substep's
 // apply and finalize and the next one's predict are one pass over the records, which are read and
-// written once, 16 bytes at a time. Bound by the record traffic (L2 for a set of this size): as
-// passes of their own with 4-byte accesses at the record's 96-byte stride, 326,800 particles took 20 (predict)
-// + 15 (apply) + 17 us (finalize) a substep; a step of two substeps 127.5 us, now 81.9.
+// written once, 16 bytes at a time. Bound by the record traffic (L2 for a set of 326,800 particles): a step of two
+// substeps takes 82 us, as passes of their own with 4-byte accesses at the record's 96-byte stride 127.5 (20 predict, 15 apply,
+// 17 finalize a substep).
 template <bool kTail, bool kHead>
 __global__ void __launch_bounds__(kSolveThreads) k_pbd_move(const SolveDev* __restrict__ sd) {
   const SolveDev& S = *sd;
