@@ -193,3 +193,37 @@ def test_gathered_surface_of_many_chunks_equals_splatted(root):
     assert (ad != 0x3C00).any()
     for o in [b, alone] + together:
         o.destroy()
+
+
+def test_choice_under_capture(root):
+    """A frame that may choose, captured by the caller: the branch joins the captured stream, and replays equal plain frames
+    where the device gathers and where it splats."""
+    import torch
+
+    import clay_engine_b200 as ce
+
+    n = 1 << 18
+    cloud = mist(n, 0.2, (0.0, 6.0, 0.0), 1)
+    far = cloud.copy()
+    far["pos"][::2] = np.random.default_rng(2).uniform((-11, -3, -11), (11, 19, 11), (n // 2, 3))
+    assert is_gathered(cloud, 64) and not is_gathered(far, 64)
+    captured, plain = surface_sim(root, cloud, 64, 2), surface_sim(root, cloud, 64, 2)
+    stream = torch.cuda.Stream()
+    captured.step(stream.cuda_stream)  # uploads what the frame reads
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        captured.step(torch.cuda.current_stream().cuda_stream)
+    for p in (cloud, far):
+        captured.upload(p)
+        plain.upload(p)
+        torch.cuda.synchronize()
+        graph.replay()
+        plain.step()
+        torch.cuda.synchronize()
+        assert np.array_equal(captured.download()["pos"], plain.download()["pos"])
+        gd, ad = captured.surface.volume.download()[0], plain.surface.volume.download()[0]
+        assert np.array_equal(gd, ad) and (ad != 0x3C00).any()
+    del graph
+    for o in (captured, plain):
+        o.destroy()
