@@ -854,19 +854,42 @@ __global__ void k_scan_partial(const SceneDev* __restrict__ scenes, const Work* 
   uint32_t beg, end;
   scan_part(S, w.sub, n, beg, end);
   if (beg >= end) return;  // part 0 always has a cell
-  uint32_t s = 0;
-  for (uint32_t c = beg + 4u * threadIdx.x; c < end; c += 4u * blockDim.x) {
-    const uint4 v = scan_counts(S, c, end);
-    s += (v.x + v.y) + (v.z + v.w);
+  // for bake_gathers, where the scene may be gathered: the cells that hold a particle (those outside the grid count as one
+  // more) and the runs of 128 cells, a warp's, that do
+  const bool census = substep + 1 == S.substeps && work_count(S) >= (work ? kGatherMin : kGatherAlone);
+  uint32_t s = 0, occupied = 0, runs = 0;
+  for (uint32_t c0 = beg; c0 < end; c0 += 4u * blockDim.x) {
+    const uint32_t c = c0 + 4u * threadIdx.x;
+    const uint4 v = c < end ? scan_counts(S, c, end) : make_uint4(0u, 0u, 0u, 0u);
+    const uint32_t sum = (v.x + v.y) + (v.z + v.w);
+    s += sum;
+    if (census) {
+      occupied += (v.x != 0u) + (v.y != 0u) + (v.z != 0u) + (v.w != 0u);
+      runs += __any_sync(0xffffffffu, sum != 0u);
+    }
   }
   s = __reduce_add_sync(0xffffffffu, s);
-  __shared__ uint32_t red[32];
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __shared__ uint32_t red[32], red_occupied[32], red_runs[32];
+  if (census) occupied = __reduce_add_sync(0xffffffffu, occupied);
+  if ((threadIdx.x & 31) == 0) {
+    red[threadIdx.x >> 5] = s;
+    red_occupied[threadIdx.x >> 5] = occupied;
+    red_runs[threadIdx.x >> 5] = runs;
+  }
   __syncthreads();
   if (threadIdx.x < 32) {
-    uint32_t v = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0u;
-    v = __reduce_add_sync(0xffffffffu, v);
+    const bool has = threadIdx.x < (blockDim.x >> 5);
+    const uint32_t v = __reduce_add_sync(0xffffffffu, has ? red[threadIdx.x] : 0u);
     if (threadIdx.x == 0) gs->part_sum[w.sub] = v;
+    if (census) {
+      occupied = __reduce_add_sync(0xffffffffu, has ? red_occupied[threadIdx.x] : 0u);
+      runs = __reduce_add_sync(0xffffffffu, has ? red_runs[threadIdx.x] : 0u);
+      if (threadIdx.x == 0 && occupied) {
+        atomicAdd(&gs->occupied, occupied);
+        atomicAdd(&gs->runs, runs);
+      }
+      if (threadIdx.x == 0 && end == n) gs->outside = S.counts[n - 1u];
+    }
   }
   if (w.sub == 0 && threadIdx.x < 6) {
     if (threadIdx.x < 3) gs->lo[threadIdx.x] = 0xffffffffu;
@@ -875,7 +898,7 @@ __global__ void k_scan_partial(const SceneDev* __restrict__ scenes, const Work* 
 }
 
 // Cell build, pass 3b: exclusive scan into cell_start[0 .. L+1], counts cleared behind.
-__global__ void __launch_bounds__(1024, 2) k_scan_final(const SceneDev* __restrict__ scenes, const Work* __restrict__ work, int substep) {
+__global__ void k_scan_final(const SceneDev* __restrict__ scenes, const Work* __restrict__ work, int substep) {
   Work w = get_work(work);
   const SceneDev& S = scenes[w.obj];
   if (substep >= S.substeps) return;
@@ -886,7 +909,7 @@ __global__ void __launch_bounds__(1024, 2) k_scan_final(const SceneDev* __restri
   scan_part(S, w.sub, n, beg, end);
   if (beg >= end) return;
   __shared__ uint32_t s_off;
-  __shared__ uint32_t s_warp[32], s_runs[32];
+  __shared__ uint32_t s_warp[32];
   if (threadIdx.x < 32) {
     uint32_t o = 0;
     for (uint32_t q = threadIdx.x; q < w.sub; q += 32u) o += gs->part_sum[q];
@@ -894,14 +917,12 @@ __global__ void __launch_bounds__(1024, 2) k_scan_final(const SceneDev* __restri
     if (threadIdx.x == 0) s_off = o;
   }
   __syncthreads();
-  uint32_t run = s_off, occupied = 0, runs = 0;
+  uint32_t run = s_off;
   const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (uint32_t c0 = beg; c0 < end; c0 += 4u * blockDim.x) {
     const uint32_t c = c0 + 4u * threadIdx.x;
     const uint4 q = c < end ? scan_counts(S, c, end) : make_uint4(0u, 0u, 0u, 0u);
     const uint32_t v = (q.x + q.y) + (q.z + q.w);
-    occupied += (q.x != 0u) + (q.y != 0u) + (q.z != 0u) + (q.w != 0u);
-    runs += __any_sync(0xffffffffu, v != 0u);
     uint32_t x = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -938,19 +959,6 @@ __global__ void __launch_bounds__(1024, 2) k_scan_final(const SceneDev* __restri
     run += tot;
   }
   if (end == n && threadIdx.x == 0) S.cell_start[n] = run;
-  // for bake_gathers: the occupied cells (with the particles outside the grid as one more)
-  if (substep + 1 == S.substeps && work_count(S) >= (work ? kGatherMin : kGatherAlone)) {
-    s_warp[wid] = __reduce_add_sync(0xffffffffu, occupied);
-    s_runs[wid] = runs;
-    __syncthreads();
-    if (wid == 0) {
-      const uint32_t all = __reduce_add_sync(0xffffffffu, lane < nw ? s_warp[lane] : 0u);
-      const uint32_t held = __reduce_add_sync(0xffffffffu, lane < nw ? s_runs[lane] : 0u);
-      if (lane == 0 && all) atomicAdd(&S.gs->occupied, all);
-      if (lane == 0 && held) atomicAdd(&S.gs->runs, held);
-      if (lane == 0 && end == n) S.gs->outside = run - S.cell_start[n - 1u];
-    }
-  }
 }
 
 // Cell build, pass 4: provisional placement.
