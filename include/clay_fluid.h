@@ -374,7 +374,8 @@ int clay_fluid_spawn(clay_fluid* sim, int64_t n, const double pos[3], const doub
                      const double* spread);
 /* FluidSim.configure (fluid.ts:528-530). `mask` = CLAY_P_* bits naming patched fields. */
 int clay_fluid_configure(clay_fluid* sim, const clay_fluid_params* patch, uint32_t mask);
-/* FluidSim.step (fluid.ts:536-558): emit, substeps, bake, enqueued on `stream`. */
+/* FluidSim.step (fluid.ts:536-558): emit, substeps, bake, enqueued on `stream` (a scene of 2^18
+ * particles and more also on a stream of its own, forked from `stream` and joined to it). */
 int clay_fluid_step(clay_fluid* sim, void* stream);
 /* FluidSim.particleCount (fluid.ts:496-498). */
 int64_t clay_fluid_particle_count(const clay_fluid* sim);

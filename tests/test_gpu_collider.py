@@ -136,3 +136,14 @@ def test_build_brush_counts_are_bit_exact(root, oracle, n, res):
     assert (gd == od).all(), f"{(gd != od).sum()} distance texels differ"
     assert (gm == om).all()
     v.destroy()
+
+
+@pytest.mark.parametrize("n", [31, 32, 34])
+def test_build_brushes_of_the_first_warp_are_bit_exact(root, oracle, n):
+    """Up to 32 brushes are culled by the first warp alone, without the count over warps: around that number."""
+    from clay_engine_b200 import scenes
+
+    v, gd, gm, od, om = build_both(root, oracle, scenes.random_brushes(n, seed=n, radius=(2.0, 6.0)), 32)
+    assert (gd == od).all(), f"{(gd != od).sum()} distance texels differ"
+    assert (gm == om).all()
+    v.destroy()
