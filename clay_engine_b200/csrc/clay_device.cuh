@@ -1761,7 +1761,7 @@ __device__ __forceinline__ uint32_t enc_key(float sd, float bw) {
 // those runs of 128 that hold any (the box of a pool under a falling stream is mostly air).
 // Measured over pools with a share of spray from none to nine tenths, without and with a stream, clouds, balls, columns,
 // layers, blobs far apart, a pool with a spray up to the sky, on 32^3 to 192^3: scenes of 262,144 to 1,000,000 by themselves
-// are gathered 1.25 times faster on average (0.94 at worst: one layer, 119 a cell), those left to the splat would
+// are gathered 1.28 times faster on average (0.94 at worst: one layer, 119 a cell), those left to the splat would
 // take up to 2.9 times as long by the gather (a pool of 259,000 and 2,600 in the sky, 192^3: 699 -> 2,000 us). In batches
 // of 393,216 and more 1.19 times (0.96 at worst). Particles outside the grid are in no order (one bin), and 7 % of them took a
 // cloud of 600,000 from 1,930 to 2,930 us: more than 1 in 64 are splatted.
